@@ -735,6 +735,27 @@ int vh_device_math_check(int which, const double *a, const double *b, int n, dou
     return VH_OK;
 }
 
+/* the branch-free square root, reciprocal and quotient (vh_math.cuh) beside
+ * the compiler's, n of each: out holds 2 n doubles */
+int vh_device_round_check(int which, const double *a, const double *b, int n, double *out)
+{
+    if (which < 0 || which > 2 || n < 1 || !a || !out || (which == 2 && !b)) return fail(VH_ERR_ARG, "bad argument");
+    if (!vh_device_available()) return fail(VH_ERR_NODEVICE, "no CUDA device");
+    double *d = nullptr;
+    const size_t B = (size_t)n * sizeof(double);
+    CUDA_TRY(cudaMalloc(&d, 4 * B));
+    cudaError_t e = cudaMemcpy(d, a, B, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && b) e = cudaMemcpy(d + n, b, B, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        vh::launch_round_check(which, d, d + n, n, d + 2 * (size_t)n, 0);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(out, d + 2 * (size_t)n, 2 * B, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    if (e != cudaSuccess) return fail(VH_ERR_CUDA, std::string("vh_device_round_check: ") + cudaGetErrorString(e));
+    return VH_OK;
+}
+
 /* ------------------------------------------------- Cornelius service */
 int vh_cornelius_surfaces(int dim, const double *cubes, int n_cubes, double value0, const double *dx,
                           double *elements, int cap_elements, int *counts, int *n_elements)

@@ -109,6 +109,12 @@ static inline vh::DevEos dev_eos(const vh_event *ev)
     E.e_spacing = ev->heos.e_spacing;
     E.inv_spacing = 1.0 / ev->heos.e_spacing;
     E.cs2_third_hi = (ev->cfg.eos_kind == VH_EOS_TABLE && !vh_env_off("VH_CS2_SHORTCUT")) ? ev->heos.cs2_third_hi : -INFINITY;
+    /* flow_pair's range argument for the table lookups (VH_CS2_SHORTCUT=0
+     * leaves every lookup to the plain root solve) */
+    auto ranged = [](double x) { return x >= 0x1p-100 && x < 0x1p100; };
+    E.direct = ev->cfg.eos_kind == VH_EOS_TABLE
+                   ? (E.cs2_third_hi > 0 && ranged(E.e_spacing) && (E.e_min == 0 || ranged(E.e_min)))
+                   : 1;
     E.pq.keys = ev->powf.keys;
     E.pq.vals = ev->powf.vals;
     E.pq.bucket = ev->powf.bucket;

@@ -84,6 +84,7 @@ struct VortArgs {
 };
 void launch_vorticity(const VortArgs &a, cudaStream_t s);
 void launch_math_check(int which, const double *a, const double *b, int n, double *out, const PowfTab &pq, cudaStream_t s);
+void launch_round_check(int which, const double *a, const double *b, int n, double *out, cudaStream_t s);
 /* Optional per-phase timing marks of one stage: ev[0] is recorded before the
  * first kernel, ev[n+1] after kernel n, whose phase id is phase[n]
  * (0 source, 1-3 x/y/eta flux, 4 finalize, 5 fused stage). */

@@ -164,6 +164,32 @@ void launch_math_check(int which, const double *a, const double *b, int n, doubl
     math_check_kernel<<<(n + 255) / 256, 256, 0, s>>>(which, a, b, n, out, pq);
 }
 
+/* the branch-free operations of vh_math.cuh against the compiler's: 0 sqrt_rn
+ * of float(a), 1 rcp_rn(a), 2 div_rn(a, b, rcp_rn(b)); out[n + i] holds the
+ * plain result */
+__global__ void round_check_kernel(int which, const double *a, const double *b, int n, double *out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double x = a[i];
+    if (which == 0) {
+        const float f = __double2float_rn(x);
+        out[i] = (double)sqrt_rn(f);
+        out[n + i] = (double)sqrtf(f);
+    } else if (which == 1) {
+        out[i] = rcp_rn(x);
+        out[n + i] = 1.0 / x;
+    } else {
+        out[i] = div_rn(x, b[i], rcp_rn(b[i]));
+        out[n + i] = x / b[i];
+    }
+}
+
+void launch_round_check(int which, const double *a, const double *b, int n, double *out, cudaStream_t s)
+{
+    round_check_kernel<<<(n + 255) / 256, 256, 0, s>>>(which, a, b, n, out);
+}
+
 __global__ void scatter_interior_kernel(const double *in, double *out, int nplanes, long long L, int nx, int ny, int nz,
                                         int ncx, int ncy)
 {

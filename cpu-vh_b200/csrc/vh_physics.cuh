@@ -26,6 +26,7 @@ struct DevEos {
     double e_min, e_spacing;
     double inv_spacing;       /* RN(1/e_spacing), for div_rcp */
     double cs2_third_hi;      /* eos_cs2 is exactly 1/3 for e <= this (HostEos::cs2_third_bound) */
+    int direct;               /* the table's e_min and e_spacing lie where flow_pair's divisions are exact */
     PowfTab pq;               /* host-exact powf(x, 0.25) */
     const int *stop;          /* the event's device error code (or null): see e_bisect_table */
 };
@@ -246,6 +247,138 @@ __device__ __forceinline__ Prim infer(const DevEos &E, double t, double M0, doub
     r.un = M3 * E2;
     if (r.ut > 1.0e3) { r.ut = 1.0; r.ux = 0.0; r.uy = 0.0; r.un = 0.0; }
     return r;
+}
+
+/* ------------------------------------------------------------------
+ * The same inversion for the two half-site states of a face, side by side and
+ * without the divisions' branches (rcp_rn, div_rn, sqrt_rn): what a flux needs
+ * of each state is u^tau, one velocity component and RN(1/u^tau).  Two
+ * independent Newton chains per thread overlap where one leaves the FP64 pipe
+ * idle between dependent operations.  Every value is e_newton_iter's and
+ * infer's, in their operation order, and every quotient is the correctly
+ * rounded one, so the result has infer's bits; where an operand leaves the
+ * range the exactness needs (or a table has no cs2_third_hi), flow_pair
+ * returns false and the caller runs infer.
+ * ------------------------------------------------------------------ */
+struct Flow { double ut, v, y; };       /* u^tau, u^dir, RN(1/u^tau) */
+
+__device__ __forceinline__ double eos_interp_direct(const DevEos &E, double ed, const double *tb)
+{
+    /* ed - e_min and ed minus a node are 0 or far above 2^-900 for ed >=
+     * 2^-100 and a table whose e_min is 0 or at least 2^-100 */
+    int idx = (int)div_rn(ed - E.e_min, E.e_spacing, E.inv_spacing);
+    idx = (E.e_length - 2 < idx) ? E.e_length - 2 : idx;
+    idx = (idx < 0) ? 0 : idx;
+    const double frac = div_rn(ed - (idx * E.e_spacing + E.e_min), E.e_spacing, E.inv_spacing);
+    return __ldg(tb + idx) * (1. - frac) + __ldg(tb + idx + 1) * frac;
+}
+
+template <int EOS>
+__device__ __forceinline__ bool flow_pair(const DevEos &E, double t, const double (&M0)[2], const double (&M1)[2],
+                                          const double (&M2)[2], const double (&M3)[2], const double (&Pi)[2], int dir,
+                                          double ePrev, Flow (&out)[2])
+{
+    double M[2], ef[2];
+    bool ok = true;
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        M[s] = M1[s] * M1[s] + M2[s] * M2[s] + t * t * M3[s] * M3[s];
+        ok = ok && in_range(M0[s]);
+    }
+    if (ePrev <= 0.1) {
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            ok = ok && rcp_ok(M0[s]) && div_key(M[s]) >= kDivKeyLo;
+            ef[s] = M0[s] - div_rn(M[s], M0[s], rcp_rn(M0[s]));
+        }
+    } else if (EOS == 0) {
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const float h2 = fabsf(__double2float_rn(4 * M0[s] * M0[s] - 3 * M[s]));
+            ok = ok && in_range(h2);
+            ef[s] = (double)fabsf(__double2float_rn((double)sqrt_rn(h2) - M0[s]));
+        }
+    } else {
+        double e0[2] = {ePrev, ePrev}, B[2];
+        bool done[2] = {false, false};
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            B[s] = M0[s] * (M0[s] + Pi[s]) - M[s];
+            ok = ok && fabs(Pi[s]) < 1e30;
+            ef[s] = ePrev;
+        }
+        const double cs2 = 1. / 3.;
+        for (int j = 0; ok; ++j) {
+            if (j == 100) { ok = false; break; }
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                const double x = e0[s];
+                bool fine = in_range(x) && x <= E.cs2_third_hi && rcp_ok(x);
+                const double pp = floor15(eos_interp_direct(E, x, E.p_tb));
+                const double yx = rcp_rn(x);
+                const double cst2 = div_rn(pp, x, yx);
+                const double A = M0[s] * (1.0 - cst2) + Pi[s];
+                const float h2 = fabsf(__double2float_rn(A * A + 4 * cst2 * B[s]));
+                fine = fine && in_range(h2);
+                const double H = (double)sqrt_rn(h2);
+                const double c2 = 2 * cst2, AH = A - H;
+                const double D = div_rn(AH, c2, rcp_rn(c2));
+                const double f = x + D;
+                const double g = cs2 - cst2;
+                const double w = g * cst2 * D * M0[s];
+                const double num = g * (B[s] + D * H - div_rn(w, x, yx));
+                const double den = cst2 * x * H;
+                const double fp = 1.0 - div_rn(num, den, rcp_rn(den));
+                const double q = div_rn(f, fp, rcp_rn(fp));
+                const unsigned k = min(min(div_key(AH), div_key(w)), min(div_key(num), div_key(f)));
+                fine = fine && k >= kDivKeyLo && rcp_ok(c2) && rcp_ok(den) && rcp_ok(fp) && in_range_abs(fp);
+                const double e = x - q;
+                const bool conv = (double)fabsf(__double2float_rn(e - x)) <= 1.0e-3 * (double)fabsf(__double2float_rn(e));
+                if (!done[s]) {
+                    ok = ok && fine;
+                    ef[s] = e;
+                    e0[s] = e;
+                    done[s] = conv;
+                }
+            }
+            if (done[0] && done[1]) break;
+        }
+    }
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        double e = ef[s];
+        const bool low = e < 1.e-7;               /* e and p are then set to 1e-7 */
+        ok = ok && (low || in_range(e));
+        double p = (EOS == 1) ? floor15(eos_interp_direct(E, e, E.p_tb)) : div_rn(e, 3., 1. / 3.);
+        if (low) { e = 1.e-7; p = 1.e-7; }
+        const double P = p + Pi[s], W = e + P;
+        const double Einv = rcp_rn(W);
+        const float x = fabsf(__double2float_rn((M0[s] + P) * Einv));
+        ok = ok && in_range_abs(W) && rcp_ok(W) && in_range(x);
+        double ut = (double)sqrt_rn(x), yu = rcp_rn(ut);
+        const double E2 = div_rn(Einv, ut, yu);
+        double v = ((dir == 1) ? M1[s] : (dir == 2) ? M2[s] : M3[s]) * E2;
+        if (ut > 1.0e3) { ut = 1.0; v = 0.0; yu = 1.0; }
+        out[s].ut = ut;
+        out[s].v = v;
+        out[s].y = yu;
+    }
+    return ok;
+}
+
+/* flow_pair's two states through infer, one after the other */
+template <int EOS>
+static __device__ __noinline__ void flow_pair_plain(const DevEos &E, double t, const double (&M0)[2], const double (&M1)[2],
+                                                    const double (&M2)[2], const double (&M3)[2], const double (&Pi)[2],
+                                                    int dir, double ePrev, Flow (&out)[2], bool &bad)
+{
+#pragma unroll 1
+    for (int s = 0; s < 2; ++s) {
+        const Prim P = infer<EOS>(E, t, M0[s], M1[s], M2[s], M3[s], Pi[s], ePrev, bad);
+        out[s].ut = P.ut;
+        out[s].v = (dir == 1) ? P.ux : (dir == 2) ? P.uy : P.un;
+        out[s].y = 1.0 / P.ut;
+    }
 }
 
 /* --------------------------------------------------- bulk viscosity */

@@ -437,6 +437,28 @@ struct FluxLines {
     }
 };
 
+template <int V>
+struct IntC { static constexpr int value = V; };
+
+/* approx_deriv(th, x, y, z) / 2 with the three differences' common sign taken
+ * from their sign bits and the minimum of their magnitudes from their bit
+ * patterns (which order as the magnitudes do): all negative -> -m/2, none
+ * negative -> m/2, else +0.  A difference of -0 counts as negative here and
+ * not there, but then m = 0 and both give +0 (the FMA adds +0).  A NaN loses
+ * against a number in the integer minimum, as in fmin.  (With infinite
+ * differences of opposite sign approx_deriv gives NaN and this 0 or NaN; the
+ * state is then no state: its root solve raises the error either way.) */
+__device__ __forceinline__ double half_slope(double th, double x, double y, double z)
+{
+    const double l = th * (y - x), c = (z - x) / 2.0, r = th * (z - y);
+    const long long il = __double_as_longlong(l), ic = __double_as_longlong(c), ir = __double_as_longlong(r);
+    const long long msk = 0x7fffffffffffffffLL;
+    const long long m = min(il & msk, min(ic & msk, ir & msk));
+    const int hl = (int)(il >> 32), hc = (int)(ic >> 32), hr = (int)(ir >> 32);
+    const int hi = ((hl & hc & hr) < 0) ? (int)0xbfe00000 : ((hl | hc | hr) >= 0) ? 0x3fe00000 : 0;
+    return fma(__longlong_as_double(m), __hiloint2double(hi, 0), 0.0);
+}
+
 /* blk: the block's index among the event's line blocks (runs blk * PB on) */
 /* the face-once flux's line bundles (mixed precision): 8 adjacent x-columns
  * along y and eta (a warp's loads are 4 rows of 64 bytes; 4 columns, 8 rows
@@ -444,6 +466,11 @@ struct FluxLines {
 template <int DIR>
 using FaceLinesG = FluxLines<DIR, (DIR == 1) ? VH_FLUX_XW : 8>;
 
+/* What bounds it: a warp's FP64 work is long dependent chains (root solves,
+ * then quotients), and 20 warps per SM do not cover them.  The root solves run
+ * two states side by side (flow_pair) and the components in groups without a
+ * branch per quotient; 131x131x61, one launch: 312 -> 270 us along x, 353 ->
+ * 317 along y, 355 -> 325 along eta, the same bits. */
 template <int NQ, int EOS, int DIR, int UNR = 1, bool PDL = false>
 __device__ __forceinline__ void flux_lines_block(const StageArgs &A, double *__restrict__ sm, long long blk)
 {
@@ -526,10 +553,10 @@ __device__ __forceinline__ void flux_lines_block(const StageArgs &A, double *__r
     __syncthreads();
     const double th = A.theta;
     for (int r = tid + W; r < (mlen_max - 1) * W; r += 128) {
-#pragma unroll 1
+#pragma unroll 3
         for (int n = 0; n < NQ; ++n) {
             const double *q = sm + n * PS + r;
-            hs[n * PS + r] = approx_deriv(th, q[-W], q[0], q[W]) / 2;
+            hs[n * PS + r] = half_slope(th, q[-W], q[0], q[W]);
         }
     }
     __syncthreads();
@@ -538,53 +565,83 @@ __device__ __forceinline__ void flux_lines_block(const StageArgs &A, double *__r
     constexpr int tst = W;
     const QTile qt{sm, PS};
     bool bad = false;
-    /* states m = 0..3: forward face R, L; backward face R, L */
-    double ut0 = 0, ut1 = 0, ut2 = 0, ut3 = 0, v0 = 0, v1 = 0, v2 = 0, v3 = 0;
+    /* the forward face's R and L states, then the backward face's */
+    Flow F0 = {0, 0, 0}, F1 = F0, F2 = F0, F3 = F0;
 #pragma unroll 1
-    for (int mm = 0; mm < 4; ++mm) {
-        const int o = (mm == 0) ? ts + tst : (mm == 3) ? ts - tst : ts;
-        const bool minus = (mm & 1) == 0;        /* R states subtract the half slope */
-        double st[9];
-#pragma unroll
-        for (int c = 0; c < 9; ++c) {
-            const int n = (c < 8) ? c : 14;
-            if (n >= NQ) { st[c] = 0; continue; }
-            const double qv = sm[n * PS + o], hv = hs[n * PS + o];
-            st[c] = minus ? qv - hv : qv + hv;
-        }
-        const Prim Pm = infer<EOS, true>(A.eos, A.t, st[0] - st[4], st[1] - st[5], st[2] - st[6], st[3] - st[7],
-                                         st[8], ePrev, bad);
-        const double vm = (DIR == 1) ? Pm.ux : (DIR == 2) ? Pm.uy : Pm.un;
-        if (mm == 0) { ut0 = Pm.ut; v0 = vm; }
-        else if (mm == 1) { ut1 = Pm.ut; v1 = vm; }
-        else if (mm == 2) { ut2 = Pm.ut; v2 = vm; }
-        else { ut3 = Pm.ut; v3 = vm; }
+    for (int face = 0; face < 2; ++face) {
+        const int oR = (face == 0) ? ts + tst : ts, oL = (face == 0) ? ts : ts - tst;
+        double M0[2], M1[2], M2[2], M3[2], Pi[2];
+        auto component = [&](int c, double (&M)[2]) {
+            const double *q0 = sm + c * PS, *q1 = sm + (4 + c) * PS, *h0 = hs + c * PS, *h1 = hs + (4 + c) * PS;
+            M[0] = (q0[oR] - h0[oR]) - (q1[oR] - h1[oR]);      /* R states subtract the half slope */
+            M[1] = (q0[oL] + h0[oL]) - (q1[oL] + h1[oL]);
+        };
+        component(0, M0);
+        component(1, M1);
+        component(2, M2);
+        component(3, M3);
+        Pi[0] = (NQ == 15) ? sm[14 * PS + oR] - hs[14 * PS + oR] : 0.0;
+        Pi[1] = (NQ == 15) ? sm[14 * PS + oL] + hs[14 * PS + oL] : 0.0;
+        Flow F[2];
+        if (!A.eos.direct || !flow_pair<EOS>(A.eos, A.t, M0, M1, M2, M3, Pi, DIR, ePrev, F))
+            flow_pair_plain<EOS>(A.eos, A.t, M0, M1, M2, M3, Pi, DIR, ePrev, F, bad);
+        if (face == 0) { F0 = F[0]; F1 = F[1]; } else { F2 = F[0]; F3 = F[1]; }
     }
-    /* u of the direction sources, read while the reciprocals run */
+    /* u of the direction sources */
     const double uts = __ldg(A.uin + s), uds = __ldg(A.uin + DIR * A.L + s);
-    const double y0 = 1.0 / ut0, y1 = 1.0 / ut1, y2 = 1.0 / ut2, y3 = 1.0 / ut3;
-    const double af = fmax(fabs(div_rcp(v1, ut1, y1)), fabs(div_rcp(v0, ut0, y0)));
-    const double ab = fmax(fabs(div_rcp(v3, ut3, y3)), fabs(div_rcp(v2, ut2, y2)));
+    const double af = fmax(fabs(div_rcp(F1.v, F1.ut, F1.y)), fabs(div_rcp(F0.v, F0.ut, F0.y)));
+    const double ab = fmax(fabs(div_rcp(F3.v, F3.ut, F3.y)), fabs(div_rcp(F2.v, F2.ut, F2.y)));
     const double d = (DIR == 1) ? A.dx : (DIR == 2) ? A.dy : A.dz;
     const double yd = (DIR == 1) ? A.inv_dx : (DIR == 2) ? A.inv_dy : A.inv_dz;
     double S[4];
     dir_sources_uv<NQ>(A, qt, ts, tst, uts, uds, d, DIR, S);
+    /* the quotients by u^tau and the spacing in their branch-free form
+     * (div_rn) while u^tau lies where it is exact; a group with a numerator
+     * or result out of range is evaluated again by div_rcp */
+    const bool uok = in_range(F0.ut) && in_range(F1.ut) && in_range(F2.ut) && in_range(F3.ut) && in_range(d);
     if (PDL) pdl_wait();
-#pragma unroll UNR
-    for (int n = 0; n < NQ; ++n) {
+    auto flux = [&](int n, auto quot, double s_n) {
         const double *q = sm + n * PS + ts, *h = hs + n * PS + ts;
         const double Rf = q[tst] - h[tst], Lf = q[0] + h[0], Rb = q[0] - h[0], Lb = q[-tst] + h[-tst];
-        double rf = div_rcp(v0 * Rf, ut0, y0) + div_rcp(v1 * Lf, ut1, y1) - af * (Rf - Lf);
+        double rf = quot(F0.v * Rf, F0.ut, F0.y) + quot(F1.v * Lf, F1.ut, F1.y) - af * (Rf - Lf);
         rf /= 2;
-        double rb = div_rcp(v2 * Rb, ut2, y2) + div_rcp(v3 * Lb, ut3, y3) - ab * (Rb - Lb);
+        double rb = quot(F2.v * Rb, F2.ut, F2.y) + quot(F3.v * Lb, F3.ut, F3.y) - ab * (Rb - Lb);
         rb /= 2;
         double r = -rf;
         r = r + rb;
-        r = div_rcp(r, d, yd);
-        if (n < 4) r += (n == 0) ? S[0] : (n == 1) ? S[1] : (n == 2) ? S[2] : S[3];
+        r = quot(r, d, yd);
+        if (n < 4) r += s_n;
         r *= A.dt;
-        A.qout[n * A.L + s] += r;
-    }
+        return r;
+    };
+    auto group = [&](int n0, auto count, auto first) {
+        constexpr int K = decltype(count)::value;
+        constexpr bool SRC = decltype(first)::value;
+        double r[K];
+        unsigned k = ~0u, top = 0;
+#pragma unroll
+        for (int i = 0; i < K; ++i) {
+            r[i] = flux(n0 + i, [&](double a, double bq, double y) { k = min(k, div_key(a)); return div_rn(a, bq, y); },
+                        SRC ? S[i & 3] : 0.0);
+            top = max(top, (unsigned)__double2hiint(r[i]) & 0x7fffffffu);
+        }
+        if (!(uok && k >= kDivKeyLo && top < 0x7ff00000u)) {
+#pragma unroll 1
+            for (int i = 0; i < K; ++i) {
+                const double v = flux(n0 + i, [](double a, double bq, double y) { return div_rcp(a, bq, y); },
+                                      !SRC ? 0.0 : i == 0 ? S[0] : i == 1 ? S[1] : i == 2 ? S[2] : S[3]);
+                A.qout[(n0 + i) * A.L + s] += v;
+            }
+            return;
+        }
+#pragma unroll
+        for (int i = 0; i < K; ++i) A.qout[(n0 + i) * A.L + s] += r[i];
+    };
+    group(0, IntC<4>(), IntC<1>());
+    int n = 4;
+#pragma unroll 1
+    for (; n + UNR <= NQ; n += UNR) group(n, IntC<UNR>(), IntC<0>());
+    if constexpr ((NQ - 4) % UNR != 0) group(n, IntC<(NQ - 4) % UNR>(), IntC<0>());
     if (bad) raise_error(A.err, kErrNan, s, A.step);
 }
 

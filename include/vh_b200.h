@@ -394,6 +394,11 @@ int vh_cornelius_surfaces_noalloc(int dim, const double *d_cubes, int n_cubes, d
  * (EquationOfState.cpp:196).  Host arrays of n doubles. */
 int vh_device_math_check(int which, const double *a, const double *b, int n, double *out);
 
+/* Diagnostic: the kernels' branch-free operations beside the compiler's on n
+ * operands: out[i] and out[n + i] are the two results.  which: 0 FP32 square
+ * root of float(a), 1 reciprocal of a, 2 quotient a / b (b used by 2 only). */
+int vh_device_round_check(int which, const double *a, const double *b, int n, double *out);
+
 /* Inputs seen outside the calibrated powf range since creation (diagnostic;
  * 0 means every temperature matched the host libm exactly). */
 int vh_event_powf_misses(vh_event *ev, unsigned long long *misses);
