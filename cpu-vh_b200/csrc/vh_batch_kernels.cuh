@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(kBatchFaceTX * kBatchFaceTY, 2) kt_batch_face_
  * single-event ones.  Dynamic shared memory: 2 * NQ * FluxLines::plane(nd)
  * doubles for the member with the most. */
 template <int NQ, int EOS, int DIR>
-__global__ void __launch_bounds__(128, 5) kt_batch_lines_kernel(const __grid_constant__ BatchLaunch B)
+__global__ void __launch_bounds__(128, 4) kt_batch_lines_kernel(const __grid_constant__ BatchLaunch B)
 {
     __shared__ __align__(16) StageArgs sA;
     extern __shared__ double smd[];

@@ -470,7 +470,13 @@ using FaceLinesG = FluxLines<DIR, (DIR == 1) ? VH_FLUX_XW : 8>;
  * then quotients), and 20 warps per SM do not cover them.  The root solves run
  * two states side by side (flow_pair) and the components in groups without a
  * branch per quotient; 131x131x61, one launch: 312 -> 270 us along x, 353 ->
- * 317 along y, 355 -> 325 along eta, the same bits. */
+ * 317 along y, 355 -> 325 along eta, the same bits.
+ * The update of q* is a reduction without a result (red.global.add.f64: the
+ * same IEEE sum, one per cell and component and launch), so no thread waits
+ * for the value it adds to; reading it, adding and storing cost 60-110 us of
+ * a launch, most along y and eta: 270 -> 209, 317 -> 221, 325 -> 225 us, and
+ * without those reads 4 blocks of 128 registers are faster than 5 of 96: 205,
+ * 209, 213 us. */
 template <int NQ, int EOS, int DIR, int UNR = 1, bool PDL = false>
 __device__ __forceinline__ void flux_lines_block(const StageArgs &A, double *__restrict__ sm, long long blk)
 {
@@ -521,7 +527,7 @@ __device__ __forceinline__ void flux_lines_block(const StageArgs &A, double *__r
     }
     const bool valid = bb >= 0;
     const long long s = valid ? bb + (long long)(pos + 2) * gst : 0;
-    if (valid) prefetch_flux_cell<NQ>(A, s, DIR);
+    if (valid) { prefetch_l2(A.uin + s); prefetch_l2(A.uin + DIR * A.L + s); }
     /* the root solves' start, read while the stencil is staged */
     const double ePrev = valid ? __ldg(A.ein + s) : 0.0;
     /* staging: slot l covers positions [first_l - 2, first_l + len_l + 2) of
@@ -630,12 +636,12 @@ __device__ __forceinline__ void flux_lines_block(const StageArgs &A, double *__r
             for (int i = 0; i < K; ++i) {
                 const double v = flux(n0 + i, [](double a, double bq, double y) { return div_rcp(a, bq, y); },
                                       !SRC ? 0.0 : i == 0 ? S[0] : i == 1 ? S[1] : i == 2 ? S[2] : S[3]);
-                A.qout[(n0 + i) * A.L + s] += v;
+                atomicAdd(A.qout + (n0 + i) * A.L + s, v);
             }
             return;
         }
 #pragma unroll
-        for (int i = 0; i < K; ++i) A.qout[(n0 + i) * A.L + s] += r[i];
+        for (int i = 0; i < K; ++i) atomicAdd(A.qout + (n0 + i) * A.L + s, r[i]);
     };
     group(0, IntC<4>(), IntC<1>());
     int n = 4;

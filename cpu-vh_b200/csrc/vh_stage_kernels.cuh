@@ -211,22 +211,18 @@ static void launch_flux_lines(const StageArgs &a, cudaStream_t s)
     launch_pdl(kt_flux_lines_kernel<NQ, EOS, DIR, MB, UNR>, dim3(blocks), dim3(128), bytes, s, a);
 }
 
-/* FP64 flux form of the phase-split stage: VH_FLUX_FORM=lines (default:
- * line pieces, 5 blocks per SM at 96 registers, the component loop unrolled
- * by 3), lines4 (4 blocks per SM, up to 128 registers, loop rolled), slopes
- * (32 x 4 tiles with shared half slopes) or staged (32 x 4 tiles, every cell
- * computing its own slopes).  Measured on the 131x131x61 Glauber event (ms
- * per step of the x/y/eta launches, two each): lines 0.74/0.77/0.78 (0.74/
- * 0.85/0.87 with the shared-memory carveout at its maximum, which left L1
- * 28 KB for the EoS table and the loads; 0.75/0.86/0.87 with the loop
- * rolled), lines4 0.89/0.98/0.99, slopes 0.98/1.00/1.03, staged
- * 1.10/1.09/1.12. */
+/* FP64 flux form of the phase-split stage: VH_FLUX_FORM=lines (default: line
+ * pieces, 4 blocks per SM at 128 registers, the component loop unrolled by 3),
+ * slopes (32 x 4 tiles with shared half slopes) or staged (32 x 4 tiles, every
+ * cell computing its own slopes).  Measured on the 131x131x61 Glauber event
+ * (ms per step of the x/y/eta launches, two each): lines 0.41/0.42/0.43,
+ * slopes 0.98/1.00/1.03, staged 1.10/1.09/1.12; lines at 5 blocks per SM of
+ * 96 registers 0.42/0.44/0.45. */
 static inline int flux_form()
 {
     static int f = [] {
         const char *e = getenv("VH_FLUX_FORM");
-        if (!e) return 3;
-        if (e[0] == 'l') return e[5] == '4' ? 2 : 3;
+        if (!e || e[0] == 'l') return 2;
         return (e[0] == 's' && e[1] == 't') ? 0 : 1;
     }();
     return f;
@@ -382,17 +378,11 @@ static void launch_stage_t(const StageArgs &a, cudaStream_t s, StageMarks *m)
     } else if (flux_staged() && flux_form() != 0) {
         const dim3 g3((a.nx + 31) / 32, a.ny, (a.nz + 3) / 4);
         if (flux_form() == 2) {
-            launch_flux_lines<NQ, EOS, 1, 4>(a, s);
+            launch_flux_lines<NQ, EOS, 1, 4, 3>(a, s);
             mark(1);
-            launch_flux_lines<NQ, EOS, 2, 4>(a, s);
+            launch_flux_lines<NQ, EOS, 2, 4, 3>(a, s);
             mark(2);
-            if (z) { launch_flux_lines<NQ, EOS, 3, 4>(a, s); mark(3); }
-        } else if (flux_form() == 3) {
-            launch_flux_lines<NQ, EOS, 1, 5, 3>(a, s);
-            mark(1);
-            launch_flux_lines<NQ, EOS, 2, 5, 3>(a, s);
-            mark(2);
-            if (z) { launch_flux_lines<NQ, EOS, 3, 5, 3>(a, s); mark(3); }
+            if (z) { launch_flux_lines<NQ, EOS, 3, 4, 3>(a, s); mark(3); }
         } else {
             launch_flux_slopes<NQ, EOS, 1>(a, grid, block, s);
             mark(1);
