@@ -18,7 +18,7 @@ static_assert(sizeof(StageArgs) % 8 == 0, "StageArgs is staged to shared memory 
 /* phase 0 source, 1-3 x/y/eta flux, 4 finalize, 5 fused stage; ZM (phases 4
  * and 5): 0 every member 2+1D, 1 every member 3+1D, 2 mixed (per member) */
 template <int NQ, int EOS, int PHASE, bool STAGE2, int ZM, bool MIXED>
-__global__ void __launch_bounds__(128, 4) kt_batch_kernel(const __grid_constant__ BatchLaunch B)
+__global__ void __launch_bounds__(128, PHASE == 0 && !MIXED ? 3 : 4) kt_batch_kernel(const __grid_constant__ BatchLaunch B)
 {
     __shared__ __align__(16) StageArgs sA;
     const int tid = threadIdx.x + blockDim.x * threadIdx.y;

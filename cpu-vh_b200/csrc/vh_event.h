@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 #include <cmath>
 #include <cstdlib>
+#include <cstring>
 #include <vector>
 #include "vh_b200.h"
 #include "vh_internal.h"
@@ -111,10 +112,15 @@ static inline vh::DevEos dev_eos(const vh_event *ev)
     E.cs2_third_hi = (ev->cfg.eos_kind == VH_EOS_TABLE && !vh_env_off("VH_CS2_SHORTCUT")) ? ev->heos.cs2_third_hi : -INFINITY;
     /* flow_pair's range argument for the table lookups (VH_CS2_SHORTCUT=0
      * leaves every lookup to the plain root solve) */
-    auto ranged = [](double x) { return x >= 0x1p-100 && x < 0x1p100; };
-    E.direct = ev->cfg.eos_kind == VH_EOS_TABLE
-                   ? (E.cs2_third_hi > 0 && ranged(E.e_spacing) && (E.e_min == 0 || ranged(E.e_min)))
-                   : 1;
+    auto ranged = [](double x) { return x >= 0x1p-60 && x < 0x1p60; };
+    E.direct = 120u << 20;
+    if (ev->cfg.eos_kind == VH_EOS_TABLE) {
+        unsigned long long b;
+        std::memcpy(&b, &E.cs2_third_hi, 8);
+        const unsigned hi = (unsigned)(b >> 32), lo = (1023u - 60u) << 20;
+        if (!(E.cs2_third_hi >= 0x1p-60) || !ranged(E.e_spacing) || !(E.e_min == 0 || ranged(E.e_min))) E.direct = 0;
+        else E.direct = hi - lo < E.direct ? hi - lo : E.direct;
+    }
     E.pq.keys = ev->powf.keys;
     E.pq.vals = ev->powf.vals;
     E.pq.bucket = ev->powf.bucket;

@@ -26,7 +26,8 @@ struct DevEos {
     double e_min, e_spacing;
     double inv_spacing;       /* RN(1/e_spacing), for div_rcp */
     double cs2_third_hi;      /* eos_cs2 is exactly 1/3 for e <= this (HostEos::cs2_third_bound) */
-    int direct;               /* the table's e_min and e_spacing lie where flow_pair's divisions are exact */
+    unsigned direct;          /* flow_pair's root solve: 2^-60 <= e with a high word less than `direct` above that
+                                 of 2^-60 is below min(2^60, cs2_third_hi); 0: not for this table */
     PowfTab pq;               /* host-exact powf(x, 0.25) */
     const int *stop;          /* the event's device error code (or null): see e_bisect_table */
 };
@@ -133,6 +134,26 @@ __device__ __forceinline__ double approx_deriv(double th, double x, double y, do
     double c = (z - x) / 2.0;
     double r = th * (z - y);
     return minmod(l, minmod(c, r));
+}
+
+/* approx_deriv with the three differences' common sign taken from their sign
+ * bits and the minimum of their magnitudes from their bit patterns (which
+ * order as the magnitudes do): all negative -> -m, none negative -> m, else
+ * +0.  A difference of -0 counts as negative here and not there, but then m = 0
+ * and both give +0 (the FMA adds +0).  A NaN loses against a number in the
+ * integer minimum, as in fmin.  (With infinite differences of opposite sign
+ * approx_deriv gives NaN and this 0 or NaN; the state is then no state: its
+ * root solve raises the error either way.)  one: the high word of the factor
+ * on m, 0x3ff00000 for 1, 0x3fe00000 for 1/2 (RN(m/2) as approx_deriv / 2). */
+__device__ __forceinline__ double limited(double th, double x, double y, double z, int one)
+{
+    const double l = th * (y - x), c = (z - x) / 2.0, r = th * (z - y);
+    const long long il = __double_as_longlong(l), ic = __double_as_longlong(c), ir = __double_as_longlong(r);
+    const long long msk = 0x7fffffffffffffffLL;
+    const long long m = min(il & msk, min(ic & msk, ir & msk));
+    const int hl = (int)(il >> 32), hc = (int)(ic >> 32), hr = (int)(ir >> 32);
+    const int hi = ((hl & hc & hr) < 0) ? (one | (int)0x80000000) : ((hl | hc | hr) >= 0) ? one : 0;
+    return fma(__longlong_as_double(m), __hiloint2double(hi, 0), 0.0);
 }
 
 /* -------------------------------------------------------- inversion */
@@ -256,9 +277,9 @@ __device__ __forceinline__ Prim infer(const DevEos &E, double t, double M0, doub
  * independent Newton chains per thread overlap where one leaves the FP64 pipe
  * idle between dependent operations.  Every value is e_newton_iter's and
  * infer's, in their operation order, and every quotient is the correctly
- * rounded one, so the result has infer's bits; where an operand leaves the
- * range the exactness needs (or a table has no cs2_third_hi), flow_pair
- * returns false and the caller runs infer.
+ * rounded one, so the result has infer's bits.  M1..M3 and Pi are formed from
+ * values that pass state_ranged; where another operand leaves the range the
+ * exactness needs, flow_pair returns false and the caller runs infer.
  * ------------------------------------------------------------------ */
 struct Flow { double ut, v, y; };       /* u^tau, u^dir, RN(1/u^tau) */
 
@@ -273,56 +294,55 @@ __device__ __forceinline__ double eos_interp_direct(const DevEos &E, double ed, 
     return __ldg(tb + idx) * (1. - frac) + __ldg(tb + idx + 1) * frac;
 }
 
-template <int EOS>
-__device__ __forceinline__ bool flow_pair(const DevEos &E, double t, const double (&M0)[2], const double (&M1)[2],
-                                          const double (&M2)[2], const double (&M3)[2], const double (&Pi)[2], int dir,
-                                          double ePrev, Flow (&out)[2])
+/* the energy density of N states (e_from_conserved, or infer's closed form
+ * below ePrev = 0.1); M = M1^2 + M2^2 + t^2 M3^2 */
+template <int EOS, int N>
+__device__ __forceinline__ bool energy_direct(const DevEos &E, const double (&M0)[N], const double (&M)[N],
+                                              const double (&Pi)[N], double ePrev, double (&ef)[N])
 {
-    double M[2], ef[2];
     bool ok = true;
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-        M[s] = M1[s] * M1[s] + M2[s] * M2[s] + t * t * M3[s] * M3[s];
-        ok = ok && in_range(M0[s]);
-    }
+    for (int s = 0; s < N; ++s) ok = ok && within<-60, 60>(M0[s]);
     if (ePrev <= 0.1) {
 #pragma unroll
-        for (int s = 0; s < 2; ++s) {
-            ok = ok && rcp_ok(M0[s]) && div_key(M[s]) >= kDivKeyLo;
+        for (int s = 0; s < N; ++s) {
+            ok = ok && rcp_ok(M0[s]);
             ef[s] = M0[s] - div_rn(M[s], M0[s], rcp_rn(M0[s]));
         }
     } else if (EOS == 0) {
 #pragma unroll
-        for (int s = 0; s < 2; ++s) {
+        for (int s = 0; s < N; ++s) {
             const float h2 = fabsf(__double2float_rn(4 * M0[s] * M0[s] - 3 * M[s]));
             ok = ok && in_range(h2);
             ef[s] = (double)fabsf(__double2float_rn((double)sqrt_rn(h2) - M0[s]));
         }
     } else {
-        double e0[2] = {ePrev, ePrev}, B[2];
-        bool done[2] = {false, false};
+        double e0[N], B[N];
+        bool done[N];
 #pragma unroll
-        for (int s = 0; s < 2; ++s) {
+        for (int s = 0; s < N; ++s) {
             B[s] = M0[s] * (M0[s] + Pi[s]) - M[s];
-            ok = ok && fabs(Pi[s]) < 1e30;
-            ef[s] = ePrev;
+            ef[s] = e0[s] = ePrev;
+            done[s] = false;
         }
         const double cs2 = 1. / 3.;
         for (int j = 0; ok; ++j) {
             if (j == 100) { ok = false; break; }
+            bool all = true;
 #pragma unroll
-            for (int s = 0; s < 2; ++s) {
+            for (int s = 0; s < N; ++s) {
                 const double x = e0[s];
-                bool fine = in_range(x) && x <= E.cs2_third_hi && rcp_ok(x);
-                const double pp = floor15(eos_interp_direct(E, x, E.p_tb));
+                bool fine = (unsigned)__double2hiint(x) - ((1023u - 60u) << 20) < E.direct && rcp_ok(x);
+                const double pp = eos_interp_direct(E, x, E.p_tb);     /* above the floor */
+                fine = fine && within<-49, 60>(pp);
                 const double yx = rcp_rn(x);
                 const double cst2 = div_rn(pp, x, yx);
                 const double A = M0[s] * (1.0 - cst2) + Pi[s];
                 const float h2 = fabsf(__double2float_rn(A * A + 4 * cst2 * B[s]));
                 fine = fine && in_range(h2);
                 const double H = (double)sqrt_rn(h2);
-                const double c2 = 2 * cst2, AH = A - H;
-                const double D = div_rn(AH, c2, rcp_rn(c2));
+                const double c2 = 2 * cst2;
+                const double D = div_rn(A - H, c2, rcp_rn(c2));
                 const double f = x + D;
                 const double g = cs2 - cst2;
                 const double w = g * cst2 * D * M0[s];
@@ -330,8 +350,7 @@ __device__ __forceinline__ bool flow_pair(const DevEos &E, double t, const doubl
                 const double den = cst2 * x * H;
                 const double fp = 1.0 - div_rn(num, den, rcp_rn(den));
                 const double q = div_rn(f, fp, rcp_rn(fp));
-                const unsigned k = min(min(div_key(AH), div_key(w)), min(div_key(num), div_key(f)));
-                fine = fine && k >= kDivKeyLo && rcp_ok(c2) && rcp_ok(den) && rcp_ok(fp) && in_range_abs(fp);
+                fine = fine && rcp_ok(c2) && rcp_ok(den) && rcp_ok(fp) && in_range_abs(fp);
                 const double e = x - q;
                 const bool conv = (double)fabsf(__double2float_rn(e - x)) <= 1.0e-3 * (double)fabsf(__double2float_rn(e));
                 if (!done[s]) {
@@ -340,23 +359,47 @@ __device__ __forceinline__ bool flow_pair(const DevEos &E, double t, const doubl
                     e0[s] = e;
                     done[s] = conv;
                 }
+                all = all && done[s];
             }
-            if (done[0] && done[1]) break;
+            if (all) break;
         }
     }
+    return ok;
+}
+
+/* infer's e, p (floored), u^tau, RN(1/u^tau) and 1/((e + P) u^tau) from the
+ * energy density; the last times M1..M3 is the velocity while u^tau <= 1e3 */
+template <int EOS>
+__device__ __forceinline__ bool flow_direct(const DevEos &E, double M0, double Pi, double &e, double &p, double &ut,
+                                            double &yu, double &E2)
+{
+    const bool low = e < 1.e-7;
+    bool ok = low || in_range(e);
+    p = (EOS == 1) ? floor15(eos_interp_direct(E, e, E.p_tb)) : div_rn(e, 3., 1. / 3.);
+    if (low) { e = 1.e-7; p = 1.e-7; }
+    const double P = p + Pi, W = e + P;
+    const double Einv = rcp_rn(W);
+    const float x = fabsf(__double2float_rn((M0 + P) * Einv));
+    ok = ok && in_range_abs(W) && rcp_ok(W) && in_range(x);
+    ut = (double)sqrt_rn(x);          /* 24 significant bits: rcp_ok */
+    yu = rcp_rn(ut);
+    E2 = div_rn(Einv, ut, yu);
+    return ok;
+}
+
+template <int EOS>
+__device__ __forceinline__ bool flow_pair(const DevEos &E, double t, const double (&M0)[2], const double (&M1)[2],
+                                          const double (&M2)[2], const double (&M3)[2], const double (&Pi)[2], int dir,
+                                          double ePrev, Flow (&out)[2])
+{
+    double M[2], ef[2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) M[s] = M1[s] * M1[s] + M2[s] * M2[s] + t * t * M3[s] * M3[s];
+    bool ok = energy_direct<EOS, 2>(E, M0, M, Pi, ePrev, ef);
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
-        double e = ef[s];
-        const bool low = e < 1.e-7;               /* e and p are then set to 1e-7 */
-        ok = ok && (low || in_range(e));
-        double p = (EOS == 1) ? floor15(eos_interp_direct(E, e, E.p_tb)) : div_rn(e, 3., 1. / 3.);
-        if (low) { e = 1.e-7; p = 1.e-7; }
-        const double P = p + Pi[s], W = e + P;
-        const double Einv = rcp_rn(W);
-        const float x = fabsf(__double2float_rn((M0[s] + P) * Einv));
-        ok = ok && in_range_abs(W) && rcp_ok(W) && in_range(x);
-        double ut = (double)sqrt_rn(x), yu = rcp_rn(ut);
-        const double E2 = div_rn(Einv, ut, yu);
+        double p, ut, yu, E2;
+        ok = flow_direct<EOS>(E, M0[s], Pi[s], ef[s], p, ut, yu, E2) && ok;
         double v = ((dir == 1) ? M1[s] : (dir == 2) ? M2[s] : M3[s]) * E2;
         if (ut > 1.0e3) { ut = 1.0; v = 0.0; yu = 1.0; }
         out[s].ut = ut;
@@ -366,13 +409,30 @@ __device__ __forceinline__ bool flow_pair(const DevEos &E, double t, const doubl
     return ok;
 }
 
+/* infer for one state in the same form; false: run infer */
+template <int EOS>
+__device__ __forceinline__ bool infer_direct(const DevEos &E, double t, double M0, double M1, double M2, double M3,
+                                             double Pi, double ePrev, Prim &r)
+{
+    const double M0s[1] = {M0}, M[1] = {M1 * M1 + M2 * M2 + t * t * M3 * M3}, Pis[1] = {Pi};
+    double ef[1], yu, E2;
+    bool ok = energy_direct<EOS, 1>(E, M0s, M, Pis, ePrev, ef);
+    r.e = ef[0];
+    ok = flow_direct<EOS>(E, M0, Pi, r.e, r.p, r.ut, yu, E2) && ok;
+    r.ux = M1 * E2;
+    r.uy = M2 * E2;
+    r.un = M3 * E2;
+    if (r.ut > 1.0e3) { r.ut = 1.0; r.ux = 0.0; r.uy = 0.0; r.un = 0.0; }
+    return ok;
+}
+
 /* flow_pair's two states through infer, one after the other */
 template <int EOS>
-static __device__ __noinline__ void flow_pair_plain(const DevEos &E, double t, const double (&M0)[2], const double (&M1)[2],
-                                                    const double (&M2)[2], const double (&M3)[2], const double (&Pi)[2],
-                                                    int dir, double ePrev, Flow (&out)[2], bool &bad)
+__device__ __forceinline__ void flow_pair_plain(const DevEos &E, double t, const double (&M0)[2], const double (&M1)[2],
+                                                const double (&M2)[2], const double (&M3)[2], const double (&Pi)[2],
+                                                int dir, double ePrev, Flow (&out)[2], bool &bad)
 {
-#pragma unroll 1
+#pragma unroll
     for (int s = 0; s < 2; ++s) {
         const Prim P = infer<EOS>(E, t, M0[s], M1[s], M2[s], M3[s], Pi[s], ePrev, bad);
         out[s].ut = P.ut;
@@ -401,12 +461,80 @@ __device__ __forceinline__ double zeta_over_s(const Zeta &Z, double T)
 __device__ __forceinline__ double dvr(double a, double b, double y) { return div_rcp(a, b, y); }
 __device__ __forceinline__ float dvr(float a, float, float y) { return a * y; }
 
+/* How a body takes its quotients: PlainQuot each by itself (div_rcp and the
+ * compiler's division in FP64, a * y in FP32); DirectQuot branch-free
+ * (div_rn, rcp_rn), collecting the range tests: when fine() is false at the
+ * end, or a result is not finite, the caller runs the body again with
+ * PlainQuot.  DirectQuot's divisors are positive (lengths, times, u^tau). */
+struct PlainQuot {
+    template <typename R>
+    __device__ __forceinline__ R operator()(R a, R b, R y) const { return dvr(a, b, y); }
+    template <typename R>
+    __device__ __forceinline__ R over(R a, R b) const { return a / b; }
+    template <typename R>
+    __device__ __forceinline__ R over_const(R a, R b, R) const { return a / b; }
+    /* as operator() where the divisor's reciprocal pays only in the other form */
+    template <typename R>
+    __device__ __forceinline__ R quotient(R a, R b, R) const { return a / b; }
+    __device__ __forceinline__ float root(float x) const { return sqrtf(x); }
+    template <typename R>
+    __device__ __forceinline__ R rcp(R b) const { return R(1.0) / b; }
+    __device__ __forceinline__ double deriv(double th, double x, double y, double z) const { return approx_deriv(th, x, y, z); }
+};
+struct DirectQuot {
+    unsigned key = ~0u;
+    bool ok = true;
+    __device__ __forceinline__ double operator()(double a, double b, double y)
+    {
+        key = min(key, div_key(a));
+        return div_rn(a, b, y);
+    }
+    __device__ __forceinline__ double rcp(double b)
+    {
+        ok = ok && in_range(b) && rcp_ok(b);
+        return rcp_rn(b);
+    }
+    __device__ __forceinline__ double over(double a, double b) { return (*this)(a, b, rcp(b)); }
+    __device__ __forceinline__ double over_const(double a, double b, double y) { return (*this)(a, b, y); }
+    __device__ __forceinline__ double quotient(double a, double b, double y) { return (*this)(a, b, y); }
+    __device__ __forceinline__ float root(float x)
+    {
+        ok = ok && in_range(x);
+        return sqrt_rn(x);
+    }
+    __device__ __forceinline__ double deriv(double th, double x, double y, double z) const { return limited(th, x, y, z, 0x3ff00000); }
+    __device__ __forceinline__ bool fine() const { return ok && key >= kDivKeyLo; }
+};
+
+/* the temperature and, where a^2 = (1/3 - cs^2)^2 vanishes, the bulk
+ * relaxation rate 15 a^2 T / (zeta/s), which is +0 whenever zeta/s > 0: the
+ * exponential and the division are then left out (the Gaussian law is
+ * positive while its exponent stays clear of underflow, the reference's law
+ * everywhere) */
+template <int EOS>
+__device__ __forceinline__ double temperature(PlainQuot &, const DevEos &E, double e) { return eos_T<EOS>(E, e); }
+template <int EOS>
+__device__ __forceinline__ double temperature(DirectQuot &dv, const DevEos &E, double e)
+{
+    dv.ok = dv.ok && in_range(e);
+    if (EOS == 1) return floor15(eos_interp_direct(E, e, E.T_tb));
+    return (double)powf_quarter(__double2float_rn(dv.over(e, E.a)), E.pq);
+}
+__device__ __forceinline__ double bulk_rate(PlainQuot &, const Zeta &Z, double a2, double T) { return 15 * a2 * T / zeta_over_s(Z, T); }
+__device__ __forceinline__ double bulk_rate(DirectQuot &dv, const Zeta &Z, double a2, double T)
+{
+    const double z = (T * 0.197326938 - Z.T0) / Z.w;
+    const bool positive = Z.law != 1 || (Z.norm >= 0x1p-100 && z * z < 600.0);
+    if (a2 == 0.0 && T > 0.0 && T < 0x1p100 && positive) return 0.0;
+    return 15 * a2 * T / zeta_over_s(Z, T);
+}
+
 /* SourceTerms.cpp:55-313, the right-hand side of the pi^{mu nu} (and Pi)
  * relaxation equations divided by u^tau.  yt = RN(1/t); every division by
  * t, 2t, t^2 and 5 goes through the shared reciprocal (dvr: the same
  * quotient in FP64, a product in FP32). */
-template <typename R, int EOS, bool BULK>
-__device__ void pimunu_rhs(const DevEos &E, const Zeta &Z, R *rhs, R t, R yt, double e_d, double p_d,
+template <typename R, int EOS, bool BULK, class Quot>
+__device__ __forceinline__ void pimunu_rhs(Quot &dv, const DevEos &E, const Zeta &Z, R *rhs, R t, R yt, double e_d, double p_d,
     double ut_d, double ux_d, double uy_d, double un_d, double utp, double uxp, double uyp, double unp,
     const R *pv, R Pi,
     R dxut, R dyut, R dnut, R dxux, R dyux, R dnux,
@@ -417,51 +545,51 @@ __device__ void pimunu_rhs(const DevEos &E, const Zeta &Z, R *rhs, R t, R yt, do
     const R delta_pipi = R(1.33333), tau_pipi = R(1.42857), delta_PiPi = R(0.666667), lambda_piPi = R(1.2);
     const R pitt = pv[0], pitx = pv[1], pity = pv[2], pitn = pv[3], pixx = pv[4];
     const R pixy = pv[5], pixn = pv[6], piyy = pv[7], piyn = pv[8], pinn = pv[9];
-    R T = R(eos_T<EOS>(E, e_d));
-    R taupiInv = T / 5 / d_etabar;
-    R beta_pi = dvr(e + p, R(5), R(0.2));
+    R T = R(temperature<EOS>(dv, E, e_d));
+    R taupiInv = dv.over(dv.over_const(T, R(5), R(0.2)), d_etabar);
+    R beta_pi = dv(e + p, R(5), R(0.2));
     R cs2 = R(eos_cs2<EOS>(E, e_d));
     R a = R(1.0) / R(3.0) - cs2;
     R a2 = a * a;
     R beta_Pi = 15 * a2 * (e + p);
-    R lambda_Pipi = dvr(8 * a, R(5), R(0.2));
+    R lambda_Pipi = dv(8 * a, R(5), R(0.2));
     R tauPiInv = R(0.0);
     /* in FP64 for both precisions: zeta/s underflows FP32 far from its peak
      * while a2 = 0 for both EoS kinds, and 0/0 must not appear */
-    if (BULK) tauPiInv = R(15 * double(a2) * double(T) / zeta_over_s(Z, double(T)));
+    if (BULK) tauPiInv = R(bulk_rate(dv, Z, double(a2), double(T)));
     R ut2 = ut * ut, un2 = un * un, t2 = t * t, t3 = t * t2;
-    const R yt2 = R(1.0) / t2, y2t = yt * R(0.5);   /* RN(1/t^2); RN(1/(2t)) = RN(1/t) / 2 */
-    const R kThird = R(1.0) / R(3.0), yut = R(1.0) / ut, ydt = R(1.0) / d_dt;
-    R dtut = dvr(R(ut_d - utp), d_dt, ydt), dtux = dvr(R(ux_d - uxp), d_dt, ydt), dtuy = dvr(R(uy_d - uyp), d_dt, ydt), dtun = dvr(R(un_d - unp), d_dt, ydt);
+    const R yt2 = dv.rcp(t2), y2t = yt * R(0.5);   /* RN(1/t^2); RN(1/(2t)) = RN(1/t) / 2 */
+    const R kThird = R(1.0) / R(3.0), yut = dv.rcp(ut), ydt = dv.rcp(d_dt);
+    R dtut = dv(R(ut_d - utp), d_dt, ydt), dtux = dv(R(ux_d - uxp), d_dt, ydt), dtuy = dv(R(uy_d - uyp), d_dt, ydt), dtun = dv(R(un_d - unp), d_dt, ydt);
     R Dut = ut * dtut + ux * dxut + uy * dyut + un * dnut + t * un * un;
     R DuxUpper = ut * dtux + ux * dxux + uy * dyux + un * dnux;
     R Dux = -DuxUpper;
     R DuyUpper = ut * dtuy + ux * dxuy + uy * dyuy + un * dnuy;
     R Duy = -DuyUpper;
-    R DunUpper = ut * dtun + ux * dxun + uy * dyun + un * dnun + dvr(2 * ut * un, t, yt);
+    R DunUpper = ut * dtun + ux * dxun + uy * dyun + un * dnun + dv(2 * ut * un, t, yt);
     R Dun = -t2 * DunUpper;
     R dut = Dut - t * un * un;
     R dux = ut * dtux + ux * dxux + uy * dyux + un * dnux;
     R duy = ut * dtuy + ux * dxuy + uy * dyuy + un * dnuy;
     R dun = ut * dtun + ux * dxun + uy * dyun + un * dnun;
-    R theta = dvr(ut, t, yt) + dtut + dxux + dyuy + dnun;
-    R stt = -t * ut * un2 + (dtut - ut * dut) + dvr((ut2 - 1) * theta, R(3.0), kThird);
-    R stx = -(t * un2 * ux) / R(2.0) + (dtux - dxut) / R(2.0) - (ux * dut + ut * dux) / R(2.0) + dvr(ut * ux * theta, R(3.0), kThird);
-    R sty = -(t * un2 * uy) / R(2.0) + (dtuy - dyut) / R(2.0) - (uy * dut + ut * duy) / R(2.0) + dvr(ut * uy * theta, R(3.0), kThird);
-    R stn = dvr(-un * (R(2.0) * ut2 + t2 * un2), R(2.0) * t, y2t) + (dtun - dvr(dnut, t2, yt2)) / R(2.0) - (un * dut + ut * dun) / R(2.0) + dvr(ut * un * theta, R(3.0), kThird);
-    R sxx = -(dxux + ux * dux) + dvr((R(1.0) + ux * ux) * theta, R(3.0), kThird);
-    R sxy = -(dxuy + dyux) / R(2.0) - (uy * dux + ux * duy) / R(2.0) + dvr(ux * uy * theta, R(3.0), kThird);
-    R sxn = dvr(-ut * ux * un, t, yt) - (dxun + dvr(dnux, t2, yt2)) / R(2.0) - (un * dux + ux * dun) / R(2.0) + dvr(ux * un * theta, R(3.0), kThird);
-    R syy = -(dyuy + uy * duy) + dvr((R(1.0) + uy * uy) * theta, R(3.0), kThird);
-    R syn = dvr(-ut * uy * un, t, yt) - (dyun + dvr(dnuy, t2, yt2)) / R(2.0) - (un * duy + uy * dun) / R(2.0) + dvr(uy * un * theta, R(3.0), kThird);
-    R snn = -ut * (R(1.0) + R(2.0) * t2 * un2) / t3 - dvr(dnun, t2, yt2) - un * dun + dvr((yt2 + un2) * theta, R(3.0), kThird);
+    R theta = dv(ut, t, yt) + dtut + dxux + dyuy + dnun;
+    R stt = -t * ut * un2 + (dtut - ut * dut) + dv((ut2 - 1) * theta, R(3.0), kThird);
+    R stx = -(t * un2 * ux) / R(2.0) + (dtux - dxut) / R(2.0) - (ux * dut + ut * dux) / R(2.0) + dv(ut * ux * theta, R(3.0), kThird);
+    R sty = -(t * un2 * uy) / R(2.0) + (dtuy - dyut) / R(2.0) - (uy * dut + ut * duy) / R(2.0) + dv(ut * uy * theta, R(3.0), kThird);
+    R stn = dv(-un * (R(2.0) * ut2 + t2 * un2), R(2.0) * t, y2t) + (dtun - dv(dnut, t2, yt2)) / R(2.0) - (un * dut + ut * dun) / R(2.0) + dv(ut * un * theta, R(3.0), kThird);
+    R sxx = -(dxux + ux * dux) + dv((R(1.0) + ux * ux) * theta, R(3.0), kThird);
+    R sxy = -(dxuy + dyux) / R(2.0) - (uy * dux + ux * duy) / R(2.0) + dv(ux * uy * theta, R(3.0), kThird);
+    R sxn = dv(-ut * ux * un, t, yt) - (dxun + dv(dnux, t2, yt2)) / R(2.0) - (un * dux + ux * dun) / R(2.0) + dv(ux * un * theta, R(3.0), kThird);
+    R syy = -(dyuy + uy * duy) + dv((R(1.0) + uy * uy) * theta, R(3.0), kThird);
+    R syn = dv(-ut * uy * un, t, yt) - (dyun + dv(dnuy, t2, yt2)) / R(2.0) - (un * duy + uy * dun) / R(2.0) + dv(uy * un * theta, R(3.0), kThird);
+    R snn = dv.over(-ut * (R(1.0) + R(2.0) * t2 * un2), t3) - dv(dnun, t2, yt2) - un * dun + dv((yt2 + un2) * theta, R(3.0), kThird);
     R wtx = (-dtux - dxut + ut * dux - ux * dut - t * un2 * ux) / R(2.0);
     R wty = (-dtuy - dyut + ut * duy - uy * dut - t * un2 * uy) / R(2.0);
     R wtn = (-t2 * dtun - R(2.0) * t * un - dnut - ut * Dun - t2 * un * dut - t3 * un * un2) / R(2.0);
     R wxy = (dxuy - dyux + ux * duy - uy * dux) / R(2.0);
     R wxn = (t2 * dxun - dnux - ux * Dun - t2 * un * dux) / R(2.0);
     R wyn = (t2 * dyun - dnuy - uy * Dun - t2 * un * duy) / R(2.0);
-    R wxt = wtx, wyt = wty, wnt = dvr(wtn, t2, yt2), wyx = -wxy, wnx = dvr(-wxn, t2, yt2), wny = dvr(-wyn, t2, yt2);
+    R wxt = wtx, wyt = wty, wnt = dv(wtn, t2, yt2), wyx = -wxy, wnx = dv(-wxn, t2, yt2), wny = dv(-wyn, t2, yt2);
     R I1tt = R(2.0) * ut * (pitt * Dut + pitx * Dux + pity * Duy + pitn * Dun);
     R I1tx = (pitt * ux + pitx * ut) * Dut + (pitx * ux + pixx * ut) * Dux + (pity * ux + pixy * ut) * Duy + (pitn * ux + pixn * ut) * Dun;
     R I1ty = (pitt * uy + pity * ut) * Dut + (pitx * uy + pixy * ut) * Dux + (pity * uy + piyy * ut) * Duy + (pitn * uy + piyn * ut) * Dun;
@@ -486,16 +614,16 @@ __device__ void pimunu_rhs(const DevEos &E, const Zeta &Z, R *rhs, R t, R yt, do
     R I3nn = R(2.0) * (pitn * wnt + pixn * wnx + piyn * wny);
     R ux2 = ux * ux, uy2 = uy * uy;
     R ps = pitt * stt - R(2.0) * pitx * stx - R(2.0) * pity * sty + pixx * sxx + R(2.0) * pixy * sxy + piyy * syy - R(2.0) * pitn * stn * t2 + R(2.0) * pixn * sxn * t2 + R(2.0) * piyn * syn * t2 + pinn * snn * t2 * t2;
-    R I4tt = (pitt * stt - pitx * stx - pity * sty - t2 * pitn * stn) - dvr((R(1.0) - ut2) * ps, R(3.0), kThird);
-    R I4tx = (pitt * stx + pitx * stt) / R(2.0) - (pitx * sxx + pixx * stx) / R(2.0) - (pity * sxy + pixy * sty) / R(2.0) - t2 * (pitn * sxn + pixn * stn) / R(2.0) + dvr((ut * ux) * ps, R(3.0), kThird);
-    R I4ty = (pitt * sty + pity * stt) / R(2.0) - (pitx * sxy + pixy * stx) / R(2.0) - (pity * syy + piyy * sty) / R(2.0) - t2 * (pitn * syn + piyn * stn) / R(2.0) + dvr((ut * uy) * ps, R(3.0), kThird);
-    R I4tn = (pitt * stn + pitn * stt) / R(2.0) - (pitx * sxn + pixn * stx) / R(2.0) - (pity * syn + piyn * sty) / R(2.0) - t2 * (pitn * snn + pinn * stn) / R(2.0) + dvr((ut * un) * ps, R(3.0), kThird);
-    R I4xx = (pitx * stx - pixx * sxx - pixy * sxy - t2 * pixn * sxn) + dvr((R(1.0) + ux2) * ps, R(3.0), kThird);
-    R I4xy = (pitx * sty + pity * stx) / R(2.0) - (pixx * sxy + pixy * sxx) / R(2.0) - (pixy * syy + piyy * sxy) / R(2.0) - t2 * (pixn * syn + piyn * sxn) / R(2.0) + dvr((ux * uy) * ps, R(3.0), kThird);
-    R I4xn = (pitx * stn + pitn * stx) / R(2.0) - (pixx * sxn + pixn * sxx) / R(2.0) - (pixy * syn + piyn * sxy) / R(2.0) - t2 * (pixn * snn + pinn * sxn) / R(2.0) + dvr((ux * un) * ps, R(3.0), kThird);
-    R I4yy = (pity * sty - pixy * sxy - piyy * syy - t2 * piyn * syn) + dvr((R(1.0) + uy2) * ps, R(3.0), kThird);
-    R I4yn = (pity * stn + pitn * sty) / R(2.0) - (pixy * sxn + pixn * sxy) / R(2.0) - (piyy * syn + piyn * syy) / R(2.0) - t2 * (piyn * snn + pinn * syn) / R(2.0) + dvr((uy * un) * ps, R(3.0), kThird);
-    R I4nn = (pitn * stn - pixn * sxn - piyn * syn - t2 * pinn * snn) + dvr((yt2 + un2) * ps, R(3.0), kThird);
+    R I4tt = (pitt * stt - pitx * stx - pity * sty - t2 * pitn * stn) - dv((R(1.0) - ut2) * ps, R(3.0), kThird);
+    R I4tx = (pitt * stx + pitx * stt) / R(2.0) - (pitx * sxx + pixx * stx) / R(2.0) - (pity * sxy + pixy * sty) / R(2.0) - t2 * (pitn * sxn + pixn * stn) / R(2.0) + dv((ut * ux) * ps, R(3.0), kThird);
+    R I4ty = (pitt * sty + pity * stt) / R(2.0) - (pitx * sxy + pixy * stx) / R(2.0) - (pity * syy + piyy * sty) / R(2.0) - t2 * (pitn * syn + piyn * stn) / R(2.0) + dv((ut * uy) * ps, R(3.0), kThird);
+    R I4tn = (pitt * stn + pitn * stt) / R(2.0) - (pitx * sxn + pixn * stx) / R(2.0) - (pity * syn + piyn * sty) / R(2.0) - t2 * (pitn * snn + pinn * stn) / R(2.0) + dv((ut * un) * ps, R(3.0), kThird);
+    R I4xx = (pitx * stx - pixx * sxx - pixy * sxy - t2 * pixn * sxn) + dv((R(1.0) + ux2) * ps, R(3.0), kThird);
+    R I4xy = (pitx * sty + pity * stx) / R(2.0) - (pixx * sxy + pixy * sxx) / R(2.0) - (pixy * syy + piyy * sxy) / R(2.0) - t2 * (pixn * syn + piyn * sxn) / R(2.0) + dv((ux * uy) * ps, R(3.0), kThird);
+    R I4xn = (pitx * stn + pitn * stx) / R(2.0) - (pixx * sxn + pixn * sxx) / R(2.0) - (pixy * syn + piyn * sxy) / R(2.0) - t2 * (pixn * snn + pinn * sxn) / R(2.0) + dv((ux * un) * ps, R(3.0), kThird);
+    R I4yy = (pity * sty - pixy * sxy - piyy * syy - t2 * piyn * syn) + dv((R(1.0) + uy2) * ps, R(3.0), kThird);
+    R I4yn = (pity * stn + pitn * sty) / R(2.0) - (pixy * sxn + pixn * sxy) / R(2.0) - (piyy * syn + piyn * syy) / R(2.0) - t2 * (piyn * snn + pinn * syn) / R(2.0) + dv((uy * un) * ps, R(3.0), kThird);
+    R I4nn = (pitn * stn - pixn * sxn - piyn * syn - t2 * pinn * snn) + dv((yt2 + un2) * ps, R(3.0), kThird);
     R Itt = I1tt + delta_pipi * I2tt - I3tt + tau_pipi * I4tt - lambda_piPi * Pi * stt;
     R Itx = I1tx + delta_pipi * I2tx - I3tx + tau_pipi * I4tx - lambda_piPi * Pi * stx;
     R Ity = I1ty + delta_pipi * I2ty - I3ty + tau_pipi * I4ty - lambda_piPi * Pi * sty;
@@ -509,26 +637,26 @@ __device__ void pimunu_rhs(const DevEos &E, const Zeta &Z, R *rhs, R t, R yt, do
     R dpitt = R(2.0) * beta_pi * stt - pitt * taupiInv - Itt - R(2.0) * un * t * pitn;
     R dpitx = R(2.0) * beta_pi * stx - pitx * taupiInv - Itx - un * t * pixn;
     R dpity = R(2.0) * beta_pi * sty - pity * taupiInv - Ity - un * t * piyn;
-    R dpitn = R(2.0) * beta_pi * stn - pitn * taupiInv - Itn - un * t * pinn - dvr(ut * pitn + un * pitt, t, yt);
+    R dpitn = R(2.0) * beta_pi * stn - pitn * taupiInv - Itn - un * t * pinn - dv(ut * pitn + un * pitt, t, yt);
     R dpixx = R(2.0) * beta_pi * sxx - pixx * taupiInv - Ixx;
     R dpixy = R(2.0) * beta_pi * sxy - pixy * taupiInv - Ixy;
-    R dpixn = R(2.0) * beta_pi * sxn - pixn * taupiInv - Ixn - dvr(ut * pixn + un * pitx, t, yt);
+    R dpixn = R(2.0) * beta_pi * sxn - pixn * taupiInv - Ixn - dv(ut * pixn + un * pitx, t, yt);
     R dpiyy = R(2.0) * beta_pi * syy - piyy * taupiInv - Iyy;
-    R dpiyn = R(2.0) * beta_pi * syn - piyn * taupiInv - Iyn - dvr(ut * piyn + un * pity, t, yt);
-    R dpinn = R(2.0) * beta_pi * snn - pinn * taupiInv - Inn - dvr(2 * (ut * pinn + un * pitn), t, yt);
-    rhs[0] = dvr(dpitt, ut, yut) + pitt * dkvk;
-    rhs[1] = dvr(dpitx, ut, yut) + pitx * dkvk;
-    rhs[2] = dvr(dpity, ut, yut) + pity * dkvk;
-    rhs[3] = dvr(dpitn, ut, yut) + pitn * dkvk;
-    rhs[4] = dvr(dpixx, ut, yut) + pixx * dkvk;
-    rhs[5] = dvr(dpixy, ut, yut) + pixy * dkvk;
-    rhs[6] = dvr(dpixn, ut, yut) + pixn * dkvk;
-    rhs[7] = dvr(dpiyy, ut, yut) + piyy * dkvk;
-    rhs[8] = dvr(dpiyn, ut, yut) + piyn * dkvk;
-    rhs[9] = dvr(dpinn, ut, yut) + pinn * dkvk;
+    R dpiyn = R(2.0) * beta_pi * syn - piyn * taupiInv - Iyn - dv(ut * piyn + un * pity, t, yt);
+    R dpinn = R(2.0) * beta_pi * snn - pinn * taupiInv - Inn - dv(2 * (ut * pinn + un * pitn), t, yt);
+    rhs[0] = dv(dpitt, ut, yut) + pitt * dkvk;
+    rhs[1] = dv(dpitx, ut, yut) + pitx * dkvk;
+    rhs[2] = dv(dpity, ut, yut) + pity * dkvk;
+    rhs[3] = dv(dpitn, ut, yut) + pitn * dkvk;
+    rhs[4] = dv(dpixx, ut, yut) + pixx * dkvk;
+    rhs[5] = dv(dpixy, ut, yut) + pixy * dkvk;
+    rhs[6] = dv(dpixn, ut, yut) + pixn * dkvk;
+    rhs[7] = dv(dpiyy, ut, yut) + piyy * dkvk;
+    rhs[8] = dv(dpiyn, ut, yut) + piyn * dkvk;
+    rhs[9] = dv(dpinn, ut, yut) + pinn * dkvk;
     if (BULK) {
         R dPi = -beta_Pi * theta - Pi * tauPiInv - delta_PiPi * Pi * theta + lambda_Pipi * ps;
-        rhs[10] = dvr(dPi, ut, yut) + Pi * dkvk;
+        rhs[10] = dv(dPi, ut, yut) + Pi * dkvk;
     }
 }
 

@@ -70,7 +70,7 @@ __device__ __forceinline__ void dir_sources(const StageArgs &A, long long s, lon
 {
     const long long L = A.L;
     const double *__restrict__ q = A.qin;
-    const double fac = 1 / d / 2;
+    const double fac = ((dir == 1) ? A.inv_dx : (dir == 2) ? A.inv_dy : A.inv_dz) / 2;
     const double ut = __ldg(A.uin + s);
     const double v = __ldg(A.uin + dir * L + s);
     const double vv = v / ut;
@@ -165,7 +165,7 @@ template <int NQ>
 __device__ __forceinline__ void dir_sources_uv(const StageArgs &A, const QTile &qt, int ts, int tst, double ut, double v,
                                                double d, int dir, double *S)
 {
-    const double fac = 1 / d / 2;
+    const double fac = ((dir == 1) ? A.inv_dx : (dir == 2) ? A.inv_dy : A.inv_dz) / 2;
     const double vv = v / ut;
 #define DER(n) ((qt(n, ts + tst) - qt(n, ts - tst)) * fac)
     const double dpitt = DER(4), dpitx = DER(5), dpity = DER(6), dpitn = DER(7);
@@ -437,28 +437,6 @@ struct FluxLines {
     }
 };
 
-template <int V>
-struct IntC { static constexpr int value = V; };
-
-/* approx_deriv(th, x, y, z) / 2 with the three differences' common sign taken
- * from their sign bits and the minimum of their magnitudes from their bit
- * patterns (which order as the magnitudes do): all negative -> -m/2, none
- * negative -> m/2, else +0.  A difference of -0 counts as negative here and
- * not there, but then m = 0 and both give +0 (the FMA adds +0).  A NaN loses
- * against a number in the integer minimum, as in fmin.  (With infinite
- * differences of opposite sign approx_deriv gives NaN and this 0 or NaN; the
- * state is then no state: its root solve raises the error either way.) */
-__device__ __forceinline__ double half_slope(double th, double x, double y, double z)
-{
-    const double l = th * (y - x), c = (z - x) / 2.0, r = th * (z - y);
-    const long long il = __double_as_longlong(l), ic = __double_as_longlong(c), ir = __double_as_longlong(r);
-    const long long msk = 0x7fffffffffffffffLL;
-    const long long m = min(il & msk, min(ic & msk, ir & msk));
-    const int hl = (int)(il >> 32), hc = (int)(ic >> 32), hr = (int)(ir >> 32);
-    const int hi = ((hl & hc & hr) < 0) ? (int)0xbfe00000 : ((hl | hc | hr) >= 0) ? 0x3fe00000 : 0;
-    return fma(__longlong_as_double(m), __hiloint2double(hi, 0), 0.0);
-}
-
 /* blk: the block's index among the event's line blocks (runs blk * PB on) */
 /* the face-once flux's line bundles (mixed precision): 8 adjacent x-columns
  * along y and eta (a warp's loads are 4 rows of 64 bytes; 4 columns, 8 rows
@@ -476,7 +454,12 @@ using FaceLinesG = FluxLines<DIR, (DIR == 1) ? VH_FLUX_XW : 8>;
  * for the value it adds to; reading it, adding and storing cost 60-110 us of
  * a launch, most along y and eta: 270 -> 209, 317 -> 221, 325 -> 225 us, and
  * without those reads 4 blocks of 128 registers are faster than 5 of 96: 205,
- * 209, 213 us. */
+ * 209, 213 us.
+ * Each thread stages its own cell's column of the stencil and the ends of a
+ * piece go to its first and last two threads (a search of the pieces per
+ * staged element before): 188, 195, 201 us.  The range test of a quotient is
+ * made once per staged value, not per quotient (state_ranged): 176, 183, 188
+ * us. */
 template <int NQ, int EOS, int DIR, int UNR = 1, bool PDL = false>
 __device__ __forceinline__ void flux_lines_block(const StageArgs &A, double *__restrict__ sm, long long blk)
 {
@@ -491,87 +474,100 @@ __device__ __forceinline__ void flux_lines_block(const StageArgs &A, double *__r
     double *__restrict__ hs = sm + NQ * PS;
     const long long sxy = (long long)A.ncx * A.ncy;
     const long long gst = (DIR == 1) ? 1 : (DIR == 2) ? (long long)A.ncx : sxy;
-    const int nxq = (A.nx + W - 1) / W;
-    const long long nbund = G::bundles(A.nx, A.ny, A.nz);
-    const long long Rtot = (long long)nd * nbund;
+    const long long Rtot = (long long)nd * G::bundles(A.nx, A.ny, A.nz);
     /* line and bundle indices in 32-bit arithmetic: an event's cell count
      * is far below 2^31 (its 61 FP64 planes alone would need 1 TB) */
     const unsigned und = (unsigned)nd;
     const long long R0 = blk * PB;
-    const long long b0 = (unsigned)R0 / und;
-    const int p0 = (int)((unsigned)R0 - (unsigned)b0 * und);
+    const unsigned b0 = (unsigned)R0 / und;
+    const int p0 = (int)((unsigned)R0 - b0 * und);
     const int tid = threadIdx.x;
-    /* padded address of bundle b's column w at position -2 along DIR, or -1
-     * if that column is outside the lattice */
-    auto base = [&](long long b, int w) -> long long {
-        if (DIR == 1) {
-            const unsigned nyq = (unsigned)(A.ny + W - 1) / W, k = (unsigned)b / nyq, jq = (unsigned)b - k * nyq;
-            const int y = (int)jq * W + w;
-            if (y >= A.ny) return -1;
-            return A.ncx * (y + 2) + sxy * (k + 2);
-        }
-        const unsigned o = (unsigned)b / (unsigned)nxq, xq = (unsigned)b - o * (unsigned)nxq;
-        const int x = (int)xq * W + w;
-        if (x >= A.nx) return -1;
-        return (DIR == 2) ? (x + 2) + sxy * (o + 2) : (x + 2) + A.ncx * (o + 2);
-    };
-    /* this thread's cell (valid: inside the lattice) */
+    /* this thread's cell (valid: inside the lattice): position pos of column w
+     * of bundle b, at shared index ts; first and left: the piece of its line in
+     * this block starts at that position and has left cells from this one on */
+    const double d = (DIR == 1) ? A.dx : (DIR == 2) ? A.dy : A.dz;
+    const double yd = (DIR == 1) ? A.inv_dx : (DIR == 2) ? A.inv_dy : A.inv_dz;
     const int w = tid % W, pr = tid / W;
-    const long long R = R0 + pr;
-    long long b = 0, bb = -1;
-    int pos = 0;
-    if (R < Rtot) {
-        b = (unsigned)R / und;
-        pos = (int)((unsigned)R - (unsigned)b * und);
-        bb = base(b, w);
+    bool valid = R0 + pr < Rtot;
+    long long s = 0;
+    int ts = 0;
+    if (valid) {
+        const unsigned R = (unsigned)R0 + (unsigned)pr, b = R / und;
+        const int pos = (int)(R - b * und);
+        if (DIR == 1) {
+            const unsigned nyq = (unsigned)(A.ny + W - 1) / W, k = b / nyq, jq = b - k * nyq;
+            const int y = (int)jq * W + w;
+            valid = y < A.ny;
+            s = A.ncx * (y + 2) + sxy * (k + 2) + (pos + 2);
+        } else {
+            const unsigned nxq = (unsigned)(A.nx + W - 1) / W, o = b / nxq, xq = b - o * nxq;
+            const int x = (int)xq * W + w;
+            valid = x < A.nx;
+            s = ((DIR == 2) ? (x + 2) + sxy * (o + 2) : (x + 2) + A.ncx * (o + 2)) + (pos + 2) * gst;
+        }
+        ts = (pr + 2 + 4 * (int)(b - b0)) * W + w;
+        if (valid) {
+            prefetch_l2(A.uin + s);
+            prefetch_l2(A.uin + DIR * A.L + s);
+            const int idx = pos - ((b == b0) ? p0 : 0), left = min(nd - pos, PB - pr);
+            /* every thread copies its own column of the stencil; the two cells
+             * before a piece are copied by its first two threads, the two after
+             * it by its last two (all four by the one thread of a single cell) */
+            auto stage = [&](int at, long long from) {
+                const double *g = A.qin + from;
+                double *d = sm + at;
+#pragma unroll 5
+                for (int n = 0; n < NQ; ++n) cp_async8(d + n * PS, g + n * A.L);
+            };
+            stage(ts, s);
+            if (idx < 2) stage(ts - 2 * W, s - 2 * gst);
+            if (left <= 2) stage(ts + 2 * W, s + 2 * gst);
+            if (idx + left == 1) { stage(ts - W, s - gst); stage(ts + W, s + gst); }
+        }
     }
-    const bool valid = bb >= 0;
-    const long long s = valid ? bb + (long long)(pos + 2) * gst : 0;
-    if (valid) { prefetch_l2(A.uin + s); prefetch_l2(A.uin + DIR * A.L + s); }
     /* the root solves' start, read while the stencil is staged */
     const double ePrev = valid ? __ldg(A.ein + s) : 0.0;
-    /* staging: slot l covers positions [first_l - 2, first_l + len_l + 2) of
-     * bundle b0 + l at shared indices [M_l, M_l + len_l + 4) */
-    const int mlen_max = PS / W;
-    for (int r = tid; r < mlen_max * W; r += 128) {
-        const int m = r / W, w = r - m * W;
-        int l = 0, M = 0, first = p0, left = PB;
-        long long off = -1;
-        for (; l < G::max_slots(nd) && left > 0; ++l) {
-            const int len = (nd - first < left) ? nd - first : left;
-            if (m < M + len + 4) {
-                if (b0 + l < nbund) {
-                    const long long bb = base(b0 + l, w);
-                    if (bb >= 0) off = bb + (long long)(first + (m - M)) * gst;
-                }
-                break;
-            }
+    cp_async_wait_all();
+    __syncthreads();
+    /* half slopes: each thread at its cell, and the NQ * 2 W positions at the
+     * two ends of every piece spread over the block */
+    const double th = A.theta;
+    bool odd = false;
+    auto slope = [&](int n, int at) {
+        const double *q = sm + n * PS + at;
+        const double x = q[-W], y = q[0], z = q[W];
+        hs[n * PS + at] = limited(th, x, y, z, 0x3fe00000);
+        return y;
+    };
+    if (valid) {
+#pragma unroll 5
+        for (int n = 0; n < NQ; ++n) odd |= !state_ranged(slope(n, ts));
+    }
+    static_assert(NQ * 2 * W <= 128, "one position per thread");
+    if (tid < NQ * 2 * W) {
+        const int n = tid / (2 * W), side = (tid / W) & 1;
+        const unsigned nq = (unsigned)((DIR == 1 ? A.ny : A.nx) + W - 1) / W, nw = (unsigned)(DIR == 1 ? A.ny : A.nx);
+        unsigned bl = b0;
+        for (int M = 0, first = p0, left = PB; left > 0; ++bl) {
+            const int len = min(nd - first, left);
+            const bool staged_col = (long long)bl * nd < Rtot && (bl % nq) * W + w < nw;
+            const int at = (side ? M + len + 2 : M + 1) * W + w;
+            const double y = slope(n, at), z = sm[n * PS + at + (side ? W : -W)];
+            if (staged_col) odd |= !state_ranged(y) || !state_ranged(z);
             M += len + 4;
             left -= len;
             first = 0;
         }
-        if (off >= 0) {
-#pragma unroll 1
-            for (int n = 0; n < NQ; ++n) cp_async8(sm + n * PS + r, A.qin + n * A.L + off);
-        }
     }
-    cp_async_wait_all();
-    __syncthreads();
-    const double th = A.theta;
-    for (int r = tid + W; r < (mlen_max - 1) * W; r += 128) {
-#pragma unroll 3
-        for (int n = 0; n < NQ; ++n) {
-            const double *q = sm + n * PS + r;
-            hs[n * PS + r] = half_slope(th, q[-W], q[0], q[W]);
-        }
-    }
-    __syncthreads();
+    /* every state of the block's cells is formed from staged values that are 0
+     * or of ordinary size: the solves and quotients below run branch-free */
+    const bool direct = !__syncthreads_or(odd) && A.eos.direct && in_range(d);
     if (!valid) return;
-    const int ts = ((int)(R - R0) + 2 + 4 * (int)(b - b0)) * W + w;
     constexpr int tst = W;
     const QTile qt{sm, PS};
     bool bad = false;
     /* the forward face's R and L states, then the backward face's */
+    bool flows = true;                       /* all four through flow_pair */
     Flow F0 = {0, 0, 0}, F1 = F0, F2 = F0, F3 = F0;
 #pragma unroll 1
     for (int face = 0; face < 2; ++face) {
@@ -589,24 +585,20 @@ __device__ __forceinline__ void flux_lines_block(const StageArgs &A, double *__r
         Pi[0] = (NQ == 15) ? sm[14 * PS + oR] - hs[14 * PS + oR] : 0.0;
         Pi[1] = (NQ == 15) ? sm[14 * PS + oL] + hs[14 * PS + oL] : 0.0;
         Flow F[2];
-        if (!A.eos.direct || !flow_pair<EOS>(A.eos, A.t, M0, M1, M2, M3, Pi, DIR, ePrev, F))
+        if (!direct || !flow_pair<EOS>(A.eos, A.t, M0, M1, M2, M3, Pi, DIR, ePrev, F)) {
+            flows = false;
             flow_pair_plain<EOS>(A.eos, A.t, M0, M1, M2, M3, Pi, DIR, ePrev, F, bad);
+        }
         if (face == 0) { F0 = F[0]; F1 = F[1]; } else { F2 = F[0]; F3 = F[1]; }
     }
     /* u of the direction sources */
     const double uts = __ldg(A.uin + s), uds = __ldg(A.uin + DIR * A.L + s);
-    const double af = fmax(fabs(div_rcp(F1.v, F1.ut, F1.y)), fabs(div_rcp(F0.v, F0.ut, F0.y)));
-    const double ab = fmax(fabs(div_rcp(F3.v, F3.ut, F3.y)), fabs(div_rcp(F2.v, F2.ut, F2.y)));
-    const double d = (DIR == 1) ? A.dx : (DIR == 2) ? A.dy : A.dz;
-    const double yd = (DIR == 1) ? A.inv_dx : (DIR == 2) ? A.inv_dy : A.inv_dz;
     double S[4];
     dir_sources_uv<NQ>(A, qt, ts, tst, uts, uds, d, DIR, S);
-    /* the quotients by u^tau and the spacing in their branch-free form
-     * (div_rn) while u^tau lies where it is exact; a group with a numerator
-     * or result out of range is evaluated again by div_rcp */
-    const bool uok = in_range(F0.ut) && in_range(F1.ut) && in_range(F2.ut) && in_range(F3.ut) && in_range(d);
     if (PDL) pdl_wait();
-    auto flux = [&](int n, auto quot, double s_n) {
+    /* component n of the update; quot(a, b, y): a / b with y = RN(1/b) */
+    double af = 0, ab = 0;
+    auto update = [&](int n, double s_n, auto quot) {
         const double *q = sm + n * PS + ts, *h = hs + n * PS + ts;
         const double Rf = q[tst] - h[tst], Lf = q[0] + h[0], Rb = q[0] - h[0], Lb = q[-tst] + h[-tst];
         double rf = quot(F0.v * Rf, F0.ut, F0.y) + quot(F1.v * Lf, F1.ut, F1.y) - af * (Rf - Lf);
@@ -618,36 +610,25 @@ __device__ __forceinline__ void flux_lines_block(const StageArgs &A, double *__r
         r = quot(r, d, yd);
         if (n < 4) r += s_n;
         r *= A.dt;
-        return r;
+        atomicAdd(A.qout + n * A.L + s, r);
     };
-    auto group = [&](int n0, auto count, auto first) {
-        constexpr int K = decltype(count)::value;
-        constexpr bool SRC = decltype(first)::value;
-        double r[K];
-        unsigned k = ~0u, top = 0;
-#pragma unroll
-        for (int i = 0; i < K; ++i) {
-            r[i] = flux(n0 + i, [&](double a, double bq, double y) { k = min(k, div_key(a)); return div_rn(a, bq, y); },
-                        SRC ? S[i & 3] : 0.0);
-            top = max(top, (unsigned)__double2hiint(r[i]) & 0x7fffffffu);
-        }
-        if (!(uok && k >= kDivKeyLo && top < 0x7ff00000u)) {
-#pragma unroll 1
-            for (int i = 0; i < K; ++i) {
-                const double v = flux(n0 + i, [](double a, double bq, double y) { return div_rcp(a, bq, y); },
-                                      !SRC ? 0.0 : i == 0 ? S[0] : i == 1 ? S[1] : i == 2 ? S[2] : S[3]);
-                atomicAdd(A.qout + (n0 + i) * A.L + s, v);
-            }
-            return;
-        }
-#pragma unroll
-        for (int i = 0; i < K; ++i) atomicAdd(A.qout + (n0 + i) * A.L + s, r[i]);
+    auto radius = [&](auto quot) {      /* the faces' spectral radii */
+        af = fmax(fabs(quot(F1.v, F1.ut, F1.y)), fabs(quot(F0.v, F0.ut, F0.y)));
+        ab = fmax(fabs(quot(F3.v, F3.ut, F3.y)), fabs(quot(F2.v, F2.ut, F2.y)));
     };
-    group(0, IntC<4>(), IntC<1>());
-    int n = 4;
+    if (flows) {
+        auto quot = [](double a, double bq, double y) { return div_rn(a, bq, y); };
+        radius(quot);
+#pragma unroll
+        for (int n = 0; n < 4; ++n) update(n, S[n], quot);
+#pragma unroll UNR
+        for (int n = 4; n < NQ; ++n) update(n, 0.0, quot);
+    } else {
+        auto quot = [](double a, double bq, double y) { return div_rcp(a, bq, y); };
+        radius(quot);
 #pragma unroll 1
-    for (; n + UNR <= NQ; n += UNR) group(n, IntC<UNR>(), IntC<0>());
-    if constexpr ((NQ - 4) % UNR != 0) group(n, IntC<(NQ - 4) % UNR>(), IntC<0>());
+        for (int n = 0; n < NQ; ++n) update(n, n == 0 ? S[0] : n == 1 ? S[1] : n == 2 ? S[2] : S[3], quot);
+    }
     if (bad) raise_error(A.err, kErrNan, s, A.step);
 }
 
@@ -680,8 +661,8 @@ __device__ __forceinline__ void flux_update(const StageArgs &A, long long s, dou
 /* SourceTerms.cpp:421-612 (USE_APPROX_DERIVATIVE; the dynamical-source arrays
  * are zero, DynamicalVariables.cpp:47-52), then Q + dt S
  * (FullyDiscreteKurganovTadmorScheme.cpp:264-273). */
-template <int NQ, int EOS>
-__device__ __forceinline__ void source_update(const StageArgs &A, long long s, double *__restrict__ acc)
+template <int NQ, int EOS, class Quot>
+__device__ __forceinline__ void source_terms(Quot &dv, const StageArgs &A, long long s, double *__restrict__ acc)
 {
     const long long L = A.L;
     const double th = A.theta;
@@ -695,42 +676,42 @@ __device__ __forceinline__ void source_update(const StageArgs &A, long long s, d
                  *__restrict__ unv = A.uin + 3 * L, *__restrict__ pv = A.pin;
     const double e = __ldg(A.ein + s), p = __ldg(pv + s);
     const double ut = __ldg(utv + s), ux = __ldg(uxv + s), uy = __ldg(uyv + s), un = __ldg(unv + s);
-    const double dxut = div_rcp(approx_deriv(th, __ldg(utv + s - sx), ut, __ldg(utv + s + sx)), A.dx, A.inv_dx);
-    const double dxux = div_rcp(approx_deriv(th, __ldg(uxv + s - sx), ux, __ldg(uxv + s + sx)), A.dx, A.inv_dx);
-    const double dxuy = div_rcp(approx_deriv(th, __ldg(uyv + s - sx), uy, __ldg(uyv + s + sx)), A.dx, A.inv_dx);
-    const double dxun = div_rcp(approx_deriv(th, __ldg(unv + s - sx), un, __ldg(unv + s + sx)), A.dx, A.inv_dx);
-    const double dyut = div_rcp(approx_deriv(th, __ldg(utv + s - sy), ut, __ldg(utv + s + sy)), A.dy, A.inv_dy);
-    const double dyux = div_rcp(approx_deriv(th, __ldg(uxv + s - sy), ux, __ldg(uxv + s + sy)), A.dy, A.inv_dy);
-    const double dyuy = div_rcp(approx_deriv(th, __ldg(uyv + s - sy), uy, __ldg(uyv + s + sy)), A.dy, A.inv_dy);
-    const double dyun = div_rcp(approx_deriv(th, __ldg(unv + s - sy), un, __ldg(unv + s + sy)), A.dy, A.inv_dy);
-    const double dnut = div_rcp(approx_deriv(th, __ldg(utv + s - sz), ut, __ldg(utv + s + sz)), A.dz, A.inv_dz);
-    const double dnux = div_rcp(approx_deriv(th, __ldg(uxv + s - sz), ux, __ldg(uxv + s + sz)), A.dz, A.inv_dz);
-    const double dnuy = div_rcp(approx_deriv(th, __ldg(uyv + s - sz), uy, __ldg(uyv + s + sz)), A.dz, A.inv_dz);
-    const double dnun = div_rcp(approx_deriv(th, __ldg(unv + s - sz), un, __ldg(unv + s + sz)), A.dz, A.inv_dz);
-    const double dxp = div_rcp(approx_deriv(th, __ldg(pv + s - sx), p, __ldg(pv + s + sx)), A.dx, A.inv_dx);
-    const double dyp = div_rcp(approx_deriv(th, __ldg(pv + s - sy), p, __ldg(pv + s + sy)), A.dy, A.inv_dy);
-    const double dnp = div_rcp(approx_deriv(th, __ldg(pv + s - sz), p, __ldg(pv + s + sz)), A.dz, A.inv_dz);
+    const double dxut = dv(dv.deriv(th, __ldg(utv + s - sx), ut, __ldg(utv + s + sx)), A.dx, A.inv_dx);
+    const double dxux = dv(dv.deriv(th, __ldg(uxv + s - sx), ux, __ldg(uxv + s + sx)), A.dx, A.inv_dx);
+    const double dxuy = dv(dv.deriv(th, __ldg(uyv + s - sx), uy, __ldg(uyv + s + sx)), A.dx, A.inv_dx);
+    const double dxun = dv(dv.deriv(th, __ldg(unv + s - sx), un, __ldg(unv + s + sx)), A.dx, A.inv_dx);
+    const double dyut = dv(dv.deriv(th, __ldg(utv + s - sy), ut, __ldg(utv + s + sy)), A.dy, A.inv_dy);
+    const double dyux = dv(dv.deriv(th, __ldg(uxv + s - sy), ux, __ldg(uxv + s + sy)), A.dy, A.inv_dy);
+    const double dyuy = dv(dv.deriv(th, __ldg(uyv + s - sy), uy, __ldg(uyv + s + sy)), A.dy, A.inv_dy);
+    const double dyun = dv(dv.deriv(th, __ldg(unv + s - sy), un, __ldg(unv + s + sy)), A.dy, A.inv_dy);
+    const double dnut = dv(dv.deriv(th, __ldg(utv + s - sz), ut, __ldg(utv + s + sz)), A.dz, A.inv_dz);
+    const double dnux = dv(dv.deriv(th, __ldg(uxv + s - sz), ux, __ldg(uxv + s + sz)), A.dz, A.inv_dz);
+    const double dnuy = dv(dv.deriv(th, __ldg(uyv + s - sz), uy, __ldg(uyv + s + sz)), A.dz, A.inv_dz);
+    const double dnun = dv(dv.deriv(th, __ldg(unv + s - sz), un, __ldg(unv + s + sz)), A.dz, A.inv_dz);
+    const double dxp = dv(dv.deriv(th, __ldg(pv + s - sx), p, __ldg(pv + s + sx)), A.dx, A.inv_dx);
+    const double dyp = dv(dv.deriv(th, __ldg(pv + s - sy), p, __ldg(pv + s + sy)), A.dy, A.inv_dy);
+    const double dnp = dv(dv.deriv(th, __ldg(pv + s - sz), p, __ldg(pv + s + sz)), A.dz, A.inv_dz);
     const double t = A.t;
     /* Tnn(e, p + Pi, un, pinn, t), EnergyMomentumTensor.cpp:328-330 */
     const double pP = p + Pi;
     const double yt = A.inv_t;
-    const double tnn = (e + pP) * un * un + div_rcp(div_rcp(pP, t, yt), t, yt) + Qv[13];
-    const double yut = 1.0 / ut;
-    const double vx = div_rcp(ux, ut, yut), vy = div_rcp(uy, ut, yut), vn = div_rcp(un, ut, yut);
-    const double dxvx = div_rcp(dxux - vx * dxut, ut, yut);
-    const double dyvy = div_rcp(dyuy - vy * dyut, ut, yut);
-    const double dnvn = div_rcp(dnun - vn * dnut, ut, yut);
+    const double tnn = (e + pP) * un * un + dv(dv(pP, t, yt), t, yt) + Qv[13];
+    const double yut = dv.rcp(ut);
+    const double vx = dv(ux, ut, yut), vy = dv(uy, ut, yut), vn = dv(un, ut, yut);
+    const double dxvx = dv(dxux - vx * dxut, ut, yut);
+    const double dyvy = dv(dyuy - vy * dyut, ut, yut);
+    const double dnvn = dv(dnun - vn * dnut, ut, yut);
     const double dkvk = dxvx + dyvy + dnvn;
     double S[NQ];
     /* the dynamical sources, SourceTerms.cpp:584-587 (0 without them) */
     const double *__restrict__ sv = A.src;
     const double s0 = sv ? __ldg(sv + s) : 0.0, s1 = sv ? __ldg(sv + L + s) : 0.0;
     const double s2 = sv ? __ldg(sv + 2 * L + s) : 0.0, s3 = sv ? __ldg(sv + 3 * L + s) : 0.0;
-    S[0] = s0 - (div_rcp(Qv[0], t, yt) + t * tnn) + dkvk * (Qv[4] - p - Pi) - vx * dxp - vy * dyp - vn * dnp;
-    S[1] = s1 - div_rcp(Qv[1], t, yt) - dxp + dkvk * Qv[5];
-    S[2] = s2 - div_rcp(Qv[2], t, yt) - dyp + dkvk * Qv[6];
-    S[3] = s3 - div_rcp(3 * Qv[3], t, yt) - dnp / A.t2pow + dkvk * Qv[7];
-    pimunu_rhs<double, EOS, NQ == 15>(A.eos, A.zeta, S + 4, t, yt, e, p, ut, ux, uy, un,
+    S[0] = s0 - (dv(Qv[0], t, yt) + t * tnn) + dkvk * (Qv[4] - p - Pi) - vx * dxp - vy * dyp - vn * dnp;
+    S[1] = s1 - dv(Qv[1], t, yt) - dxp + dkvk * Qv[5];
+    S[2] = s2 - dv(Qv[2], t, yt) - dyp + dkvk * Qv[6];
+    S[3] = s3 - dv(3 * Qv[3], t, yt) - dv.over(dnp, A.t2pow) + dkvk * Qv[7];
+    pimunu_rhs<double, EOS, NQ == 15>(dv, A.eos, A.zeta, S + 4, t, yt, e, p, ut, ux, uy, un,
                               __ldg(A.upin + s), __ldg(A.upin + L + s), __ldg(A.upin + 2 * L + s), __ldg(A.upin + 3 * L + s),
                               Qv + 4, Pi, dxut, dyut, dnut, dxux, dyux, dnux, dxuy, dyuy, dnuy, dxun, dyun, dnun, dkvk,
                               A.etabar, A.dt);
@@ -738,19 +719,34 @@ __device__ __forceinline__ void source_update(const StageArgs &A, long long s, d
     for (int n = 0; n < NQ; ++n) acc[n] = Qv[n] + A.dt * S[n];
 }
 
-/* regulateDissipativeCurrents, REG_SCHEME_1 (FullyDiscreteKurganovTadmorScheme.cpp:690-859).
- * When e > e_reg both factors are exactly 1 and the reference's multiplies are
- * identities, so the block is skipped. */
-template <int NQ>
-__device__ __forceinline__ void regulate(const StageArgs &A, double *__restrict__ acc, const Prim &P, bool &bad,
-                                         long long s)
+/* the source terms with branch-free quotients (about 90 of them, 60 with a
+ * shared divisor); false: an operand is out of their range */
+template <int NQ, int EOS>
+__device__ __forceinline__ bool source_direct(const StageArgs &A, long long s, double *__restrict__ acc)
 {
-    if (P.e > A.e_reg) {
-        /* regFacShear / regFacBulk of the reference (kept only when asked for) */
-        if (A.regfac) { A.regfac[s] = 1.0; if (NQ == 15) A.regfac[A.L + s] = 1.0; }
-        return;
-    }
-    const double t = A.t_inf, t2 = t * t;
+    DirectQuot dv;
+    dv.ok = A.eos.direct && in_range(A.t) && in_range(A.dx) && in_range(A.dy) && in_range(A.dz) && in_range(A.etabar) &&
+            in_range(2 * A.t);
+    source_terms<NQ, EOS>(dv, A, s, acc);
+    unsigned top = 0;
+#pragma unroll
+    for (int n = 0; n < NQ; ++n) top = max(top, (unsigned)__double2hiint(acc[n]) & 0x7fffffffu);
+    return dv.fine() && top < 0x7ff00000u;
+}
+template <int NQ, int EOS>
+__device__ __forceinline__ void source_update(const StageArgs &A, long long s, double *__restrict__ acc)
+{
+    PlainQuot dv;
+    source_terms<NQ, EOS>(dv, A, s, acc);
+}
+
+/* regulateDissipativeCurrents, REG_SCHEME_1 (FullyDiscreteKurganovTadmorScheme.cpp:690-859):
+ * the factors tanh(rho)/rho of pi^{mu nu} and Pi. */
+template <int NQ, class Quot>
+__device__ __forceinline__ void regulation_factors(Quot &dv, double t, const double *__restrict__ acc, const Prim &P,
+                                                   double &facShear, double &facBulk)
+{
+    const double t2 = t * t;
     const double pitt = acc[4], pitx = acc[5], pity = acc[6], pitn = acc[7], pixx = acc[8];
     const double pixy = acc[9], pixn = acc[10], piyy = acc[11], piyn = acc[12], pinn = acc[13];
     const double Pi = (NQ == 15) ? acc[14] : 0;
@@ -763,28 +759,77 @@ __device__ __forceinline__ void regulate(const StageArgs &A, double *__restrict_
     double piu1 = -(pixn * t2 * un) + pitx * ut - pixx * ux - pixy * uy;
     double piu2 = -(piyn * t2 * un) + pity * ut - pixy * ux - piyy * uy;
     double piu3 = -(pinn * t2 * un) + pitn * ut - pixn * ux - piyn * uy;
-    double a1 = spipi / rhomax / (double)sqrtf(__double2float_rn(P.e * P.e + 3 * P.p * P.p));
-    double a2 = pimumu / xi0 / rhomax / spipi;
-    double a3 = piu0 / xi0 / rhomax / spipi;
-    double a4 = piu1 / xi0 / rhomax / spipi;
-    double a5 = piu2 / xi0 / rhomax / spipi;
-    double a6 = piu3 / xi0 / rhomax / spipi;
+    /* the divisions by rhomax = 1 of the source are exact and left out */
+    static_assert(rhomax == 1.0, "");
+    const double ys = dv.rcp(spipi);
+    double a1 = dv.over(spipi, (double)dv.root(__double2float_rn(P.e * P.e + 3 * P.p * P.p)));
+    double a2 = dv.quotient(dv.over_const(pimumu, xi0, 1.0 / xi0), spipi, ys);
+    double a3 = dv.quotient(dv.over_const(piu0, xi0, 1.0 / xi0), spipi, ys);
+    double a4 = dv.quotient(dv.over_const(piu1, xi0, 1.0 / xi0), spipi, ys);
+    double a5 = dv.quotient(dv.over_const(piu2, xi0, 1.0 / xi0), spipi, ys);
+    double a6 = dv.quotient(dv.over_const(piu3, xi0, 1.0 / xi0), spipi, ys);
     double a12 = fmax(a1, a2), a34 = fmax(a3, a4), a56 = fmax(a5, a6), a3456 = fmax(a34, a56);
     double rho = fmax(a12, a3456);
-    double facShear = vh_tanh(rho) / rho;
+    auto over = [&](double a, double b) { return dv.over(a, b); };
+    facShear = dv.over(vh_tanh(rho, over), rho);
     if (fabs(rho) < 1.e-7) facShear = 1.0;
+    facBulk = 1.0;
+    if (NQ == 15) {
+        double rhoBulk = dv.over(fabs(Pi), P.p);
+        facBulk = dv.over(vh_tanh(rhoBulk, over), rhoBulk);
+        if (fabs(rhoBulk) < 1.e-7) facBulk = 1.0;
+    }
+}
+
+/* When e > e_reg both factors are exactly 1 and the reference's multiplies are
+ * identities, so the block is skipped. */
+template <int NQ, bool DIRECT = false>
+__device__ __forceinline__ void regulate(const StageArgs &A, double *__restrict__ acc, const Prim &P, bool &bad,
+                                         long long s)
+{
+    if (P.e > A.e_reg) {
+        /* regFacShear / regFacBulk of the reference (kept only when asked for) */
+        if (A.regfac) { A.regfac[s] = 1.0; if (NQ == 15) A.regfac[A.L + s] = 1.0; }
+        return;
+    }
+    double facShear, facBulk;
+    if constexpr (DIRECT) {
+        DirectQuot dv;
+        regulation_factors<NQ>(dv, A.t_inf, acc, P, facShear, facBulk);
+        if (!dv.fine() || !in_range(facShear) || !in_range(facBulk)) {
+            PlainQuot pq;
+            regulation_factors<NQ>(pq, A.t_inf, acc, P, facShear, facBulk);
+        }
+    } else {
+        PlainQuot dv;
+        regulation_factors<NQ>(dv, A.t_inf, acc, P, facShear, facBulk);
+    }
 #pragma unroll
     for (int n = 4; n < 14; ++n) acc[n] *= facShear;
     if (isnan(facShear)) bad = true;
     if (A.regfac) A.regfac[s] = facShear;
     if (NQ == 15) {
-        double rhoBulk = fabs(Pi) / P.p;
-        double facBulk = vh_tanh(rhoBulk) / rhoBulk;
-        if (fabs(rhoBulk) < 1.e-7) facBulk = 1.0;
         acc[14] *= facBulk;
         if (isnan(facBulk)) bad = true;
         if (A.regfac) A.regfac[A.L + s] = facBulk;
     }
+}
+
+/* (e, p, u) of the updated cell and its regulation, in the branch-free form
+ * where it applies */
+template <int NQ, int EOS>
+__device__ __forceinline__ Prim recover(const StageArgs &A, double *__restrict__ acc, double ePrev, bool &bad, long long s)
+{
+    const double M0 = acc[0] - acc[4], M1 = acc[1] - acc[5], M2 = acc[2] - acc[6], M3 = acc[3] - acc[7];
+    const double Pi = (NQ == 15) ? acc[14] : 0.0;
+    Prim P;
+    bool ranged = A.eos.direct != 0;
+#pragma unroll
+    for (int n = 0; n < 8; ++n) ranged = ranged && state_ranged(acc[n]);
+    if (!(ranged && state_ranged(Pi)) || !infer_direct<EOS>(A.eos, A.t_inf, M0, M1, M2, M3, Pi, ePrev, P))
+        P = infer<EOS>(A.eos, A.t_inf, M0, M1, M2, M3, Pi, ePrev, bad);
+    regulate<NQ, true>(A, acc, P, bad, s);
+    return P;
 }
 
 template <int NQ>
@@ -856,10 +901,18 @@ __device__ __forceinline__ void stage_body(const StageArgs &A, int i, int j, int
  * partial sums live in qout between phases; FP64 stores are exact, so the
  * split stage is bit-identical to stage_body. */
 template <int NQ, int EOS>
-__device__ __forceinline__ void source_body(const StageArgs &A, long long s)
+static __device__ __noinline__ void source_body_plain(const StageArgs &A, long long s)
 {
     double acc[NQ];
     source_update<NQ, EOS>(A, s, acc);
+#pragma unroll
+    for (int n = 0; n < NQ; ++n) A.qout[n * A.L + s] = acc[n];
+}
+template <int NQ, int EOS>
+__device__ __forceinline__ void source_body(const StageArgs &A, long long s)
+{
+    double acc[NQ];
+    if (!source_direct<NQ, EOS>(A, s, acc)) { source_body_plain<NQ, EOS>(A, s); return; }
 #pragma unroll
     for (int n = 0; n < NQ; ++n) A.qout[n * A.L + s] = acc[n];
 }
@@ -1013,7 +1066,8 @@ __device__ __forceinline__ void source_update_m(const StageArgs &A, long long s,
     float pvf[10];
 #pragma unroll
     for (int n = 0; n < 10; ++n) pvf[n] = (float)Qv[4 + n];
-    pimunu_rhs<float, EOS, NQ == 15>(A.eos, A.zeta, S + 4, t, yt, e, p, utd, uxd, uyd, und,
+    PlainQuot dv;
+    pimunu_rhs<float, EOS, NQ == 15>(dv, A.eos, A.zeta, S + 4, t, yt, e, p, utd, uxd, uyd, und,
                                      __ldg(A.upin + s), __ldg(A.upin + L + s), __ldg(A.upin + 2 * L + s), __ldg(A.upin + 3 * L + s),
                                      pvf, Pi, dxut, dyut, dnut, dxux, dyux, dnux, dxuy, dyuy, dnuy, dxun, dyun, dnun, dkvk,
                                      (float)A.etabar, (float)A.dt);
@@ -1352,9 +1406,14 @@ __device__ __forceinline__ void stage_faces_cell(const StageArgs &A, int i, int 
                 for (int n = 0; n < NQ; ++n) { acc[n] += __ldg(A.qbase + n * A.L + s); acc[n] /= 2; }
             }
         }
-        Prim P = infer<EOS, true>(A.eos, A.t_inf, acc[0] - acc[4], acc[1] - acc[5], acc[2] - acc[6], acc[3] - acc[7],
-                                  (NQ == 15) ? acc[14] : 0.0, ePrev, bad);
-        regulate<NQ>(A, acc, P, bad, s);
+        Prim P;
+        if constexpr (MIXED) {
+            P = infer<EOS, true>(A.eos, A.t_inf, acc[0] - acc[4], acc[1] - acc[5], acc[2] - acc[6], acc[3] - acc[7],
+                                 (NQ == 15) ? acc[14] : 0.0, ePrev, bad);
+            regulate<NQ>(A, acc, P, bad, s);
+        } else {
+            P = recover<NQ, EOS>(A, acc, ePrev, bad, s);
+        }
         put_with_ghosts<NQ>(A, i, j, k, s, acc, P);
     }
     if (bad) raise_error(A.err, kErrNan, s, A.step);

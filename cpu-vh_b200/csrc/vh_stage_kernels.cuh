@@ -13,9 +13,10 @@
 namespace vh {
 
 #ifndef VH_STAGE_MIN_BLOCKS
-#define VH_STAGE_MIN_BLOCKS 4   /* 128 registers: 16 warps/SM; measured faster than 2-3 blocks at 168-255
-                                   (the source kernel, which spills 224 bytes at 128: 0.78 ms per launch
-                                   against 0.89 at 3 blocks and 168 registers) */
+#define VH_STAGE_MIN_BLOCKS 4   /* 128 registers: 16 warps/SM; measured faster than 2-3 blocks at 168-255.  The FP64
+                                   source kernel alone runs 3 blocks: branch-free (source_direct) it is bound by
+                                   the FP64 pipe and by what 128 registers spill, 131 us per 131x131x61 launch
+                                   against 146 at 4 blocks (234 with a branch per quotient) */
 #endif
 
 /* interior cell (i, j, k) of this thread, at padded index s */
@@ -61,7 +62,7 @@ __global__ void __launch_bounds__(128, VH_STAGE_MIN_BLOCKS) kt_stage_kernel(cons
  * instruction cache: the fused kernel spends most of its stall time waiting
  * for instruction fetch on large lattices. */
 template <int NQ, int EOS, bool MIXED>
-__global__ void __launch_bounds__(128, VH_STAGE_MIN_BLOCKS) kt_source_kernel(const __grid_constant__ StageArgs A)
+__global__ void __launch_bounds__(128, MIXED ? VH_STAGE_MIN_BLOCKS : 3) kt_source_kernel(const __grid_constant__ StageArgs A)
 {
     pdl_wait();       /* reads the previous stage's results: wait, then let the flux start */
     pdl_trigger();
