@@ -565,7 +565,7 @@ int vh_event_phase_times(vh_event *ev, double *ms, long long *launches)
 int vh_event_kernel_launches(vh_event *ev, int *per_step)
 {
     if (!ev || !per_step) return fail(VH_ERR_ARG, "null argument");
-    *per_step = 2 * vh::stage_launches(ev->cfg.nx, ev->cfg.ny, ev->cfg.nz);
+    *per_step = 2 * vh::stage_launches(ev->cfg.nx, ev->cfg.ny, ev->cfg.nz, ev->cfg.precision == VH_PREC_MIXED);
     return VH_OK;
 }
 

@@ -94,7 +94,7 @@ struct StageMarks {
     int n;
 };
 void launch_stage(const StageArgs &a, int nq, int eos_kind, cudaStream_t s, StageMarks *m = nullptr);
-int stage_launches(int nx, int ny, int nz);   /* kernel launches per RK stage */
+int stage_launches(int nx, int ny, int nz, bool mixed);   /* kernel launches per RK stage */
 /* the same stage in mixed precision (vh_mixed.cu) */
 void launch_stage_mixed(const StageArgs &a, int nq, int eos_kind, cudaStream_t s, StageMarks *m = nullptr);
 

@@ -218,11 +218,9 @@ void launch_init(const InitArgs &a, cudaStream_t s)
     init_kernel<<<grid, block, 0, s>>>(a);
 }
 
-int stage_launches(int nx, int ny, int nz)
+int stage_launches(int nx, int ny, int nz, bool mixed)
 {
-    StageArgs a{};
-    a.nx = nx; a.ny = ny; a.nz = nz;
-    if (!use_split(a)) return 1;
+    if (!use_split(nx, ny, nz, mixed)) return 1;
     return nz > 1 ? 5 : 4;
 }
 

@@ -1337,6 +1337,58 @@ __device__ __forceinline__ void flux_faces_lines(const StageArgs &A, double *__r
  * is bit-identical (the backward face is accumulated onto -0.0, which leaves
  * every value, signed zeros included, unchanged).
  * --------------------------------------------------------------------- */
+/* face_flux of one face (r = -H for the forward one, H for the backward) with
+ * its two root solves side by side and branch-free quotients; false: a state
+ * is out of their range */
+template <int NQ, int EOS>
+__device__ __forceinline__ bool face_direct(const StageArgs &A, long long b, long long st, int dir, bool fwd,
+                                            double ePrev, double *__restrict__ r)
+{
+    const double th = A.theta;
+    double qR[NQ], qL[NQ];
+    bool ok = A.eos.direct != 0;
+#pragma unroll
+    for (int n = 0; n < NQ; ++n) {
+        const double *__restrict__ q = A.qin + n * A.L + b;
+        const double x = __ldg(q - st), y = __ldg(q), z = __ldg(q + st), v = __ldg(q + 2 * st);
+        qR[n] = z - limited(th, y, z, v, 0x3fe00000);
+        qL[n] = y + limited(th, x, y, z, 0x3fe00000);
+        ok = ok && half_state_ranged(qR[n]) && half_state_ranged(qL[n]);
+    }
+    const double M0[2] = {qR[0] - qR[4], qL[0] - qL[4]}, M1[2] = {qR[1] - qR[5], qL[1] - qL[5]};
+    const double M2[2] = {qR[2] - qR[6], qL[2] - qL[6]}, M3[2] = {qR[3] - qR[7], qL[3] - qL[7]};
+    const double Pi[2] = {(NQ == 15) ? qR[NQ - 1] : 0.0, (NQ == 15) ? qL[NQ - 1] : 0.0};
+    Flow F[2];
+    ok = flow_pair<EOS>(A.eos, A.t, M0, M1, M2, M3, Pi, dir, ePrev, F) && ok;
+    const double a = fmax(fabs(div_rn(F[1].v, F[1].ut, F[1].y)), fabs(div_rn(F[0].v, F[0].ut, F[0].y)));
+#pragma unroll
+    for (int n = 0; n < NQ; ++n) {
+        double res = div_rn(F[0].v * qR[n], F[0].ut, F[0].y) + div_rn(F[1].v * qL[n], F[1].ut, F[1].y) - a * (qR[n] - qL[n]);
+        res /= 2;
+        r[n] = fwd ? -res : res;
+    }
+    return ok;
+}
+
+/* the face's plain form, into its shared-memory column */
+template <int NQ, int EOS>
+static __device__ __noinline__ void face_plain(const StageArgs &A, long long b, long long st, int dir, bool fwd,
+                                               double ePrev, double *__restrict__ col, int stride, bool &bad)
+{
+    double r[NQ];
+#pragma unroll
+    for (int n = 0; n < NQ; ++n) r[n] = -0.0;
+    face_flux<NQ, EOS>(A, b, st, dir, fwd, ePrev, r, bad);
+#pragma unroll
+    for (int n = 0; n < NQ; ++n) col[n * stride] = r[n];
+}
+
+template <int NQ, int EOS>
+static __device__ __noinline__ void source_plain(const StageArgs &A, long long s, double *__restrict__ acc)
+{
+    source_update<NQ, EOS>(A, s, acc);
+}
+
 template <int NQ, int EOS, bool HAS_Z, bool STAGE2, bool MIXED>
 __device__ __forceinline__ void stage_faces_cell(const StageArgs &A, int i, int j, int k, bool valid,
                                                  double *__restrict__ sm /* [2 ndir][NQ][TX] */, int TX)
@@ -1353,15 +1405,22 @@ __device__ __forceinline__ void stage_faces_cell(const StageArgs &A, int i, int 
         const long long st = (dir == 1) ? 1 : (dir == 2) ? (long long)A.ncx : sxy;
         const double ePrev = __ldg(A.ein + s);
         double r[NQ];
+        double *col = sm + (role - 1) * NQ * TX + tx;
+        if constexpr (MIXED) {
 #pragma unroll
-        for (int n = 0; n < NQ; ++n) r[n] = -0.0;
-        if constexpr (MIXED) face_flux_m<NQ, EOS>(A, fwd ? s : s - st, st, dir, fwd, ePrev, r, bad);
-        else face_flux<NQ, EOS>(A, fwd ? s : s - st, st, dir, fwd, ePrev, r, bad);
+            for (int n = 0; n < NQ; ++n) r[n] = -0.0;
+            face_flux_m<NQ, EOS>(A, fwd ? s : s - st, st, dir, fwd, ePrev, r, bad);
 #pragma unroll
-        for (int n = 0; n < NQ; ++n) sm[((role - 1) * NQ + n) * TX + tx] = r[n];
+            for (int n = 0; n < NQ; ++n) col[n * TX] = r[n];
+        } else if (face_direct<NQ, EOS>(A, fwd ? s : s - st, st, dir, fwd, ePrev, r)) {
+#pragma unroll
+            for (int n = 0; n < NQ; ++n) col[n * TX] = r[n];
+        } else {
+            face_plain<NQ, EOS>(A, fwd ? s : s - st, st, dir, fwd, ePrev, col, TX, bad);
+        }
     } else if (valid) {
         if constexpr (MIXED) source_update_m<NQ, EOS>(A, s, acc);
-        else source_update<NQ, EOS>(A, s, acc);
+        else if (!source_direct<NQ, EOS>(A, s, acc)) source_plain<NQ, EOS>(A, s, acc);
     }
     __syncthreads();
     if (valid && role == 0) {
@@ -1383,8 +1442,16 @@ __device__ __forceinline__ void stage_faces_cell(const StageArgs &A, int i, int 
 #pragma unroll
                 for (int n = 4; n < NQ; ++n) acc[n] += r[n] * yd * A.dt;
             } else {
+                unsigned key = ~0u;
 #pragma unroll
-                for (int n = 0; n < NQ; ++n) r[n] = div_rcp(r[n], d, yd);
+                for (int n = 0; n < NQ; ++n) key = min(key, div_key(r[n]));
+                if (key >= kDivKeyLo && in_range(d)) {
+#pragma unroll
+                    for (int n = 0; n < NQ; ++n) r[n] = div_rn(r[n], d, yd);
+                } else {
+#pragma unroll
+                    for (int n = 0; n < NQ; ++n) r[n] = div_rcp(r[n], d, yd);
+                }
 #pragma unroll
                 for (int n = 0; n < 4; ++n) { r[n] += S[n]; r[n] *= A.dt; }
 #pragma unroll

@@ -82,7 +82,11 @@ __global__ void __launch_bounds__(128, VH_STAGE_MIN_BLOCKS) kt_flux_kernel(const
 }
 
 /* face-parallel fused stage (small lattices): 32 cells of one row per block,
- * 1 + 2 ndir threads per cell */
+ * 1 + 2 ndir threads per cell.  It is a latency: the longest thread's chain
+ * (a face's two root solves, or the source terms, then the cell's inversion and
+ * regulation).  With the two root solves side by side and branch-free
+ * quotients throughout (face_direct, source_direct, recover), us per stage:
+ * conformal 101^2 22.1 -> 14.4, table 161^2 69.5 -> 45.4, 41x37x21 147 -> 85. */
 constexpr int kFacesTX = 32;
 
 template <int NQ, int EOS, bool HAS_Z, bool STAGE2, bool MIXED>
@@ -90,6 +94,8 @@ __global__ void __launch_bounds__(kFacesTX * 7, 2) kt_stage_faces_kernel(const _
 {
     constexpr int ND = HAS_Z ? 3 : 2;
     __shared__ double sm[2 * ND * NQ * kFacesTX];
+    pdl_wait();       /* reads the previous stage's results */
+    pdl_trigger();
     const int i = blockIdx.x * kFacesTX + threadIdx.x + 2;
     const int j = blockIdx.y + 2;
     const int k = blockIdx.z + 2;
@@ -313,18 +319,24 @@ __global__ void __launch_bounds__(128, VH_STAGE_MIN_BLOCKS) kt_final_kernel(cons
 }
 
 /* Fused (face-parallel) for small lattices, which are latency-bound;
- * phase-split from 2^15 interior cells up.  Measured on B200 (FP64, table EoS,
- * ms/step fused vs split): 101^2 0.095 vs 0.253; 201^2 0.309 vs 0.285; 41^3
- * 1.07 vs 0.62; 131x131x61 12.98 vs 5.18.  VH_STAGE_MODE=fused|split
- * overrides. */
-static inline bool use_split(const StageArgs &a)
+ * phase-split otherwise.  FP64: fused while all its blocks are resident at
+ * once (3 per SM with the 5 warps of a 2+1D block, 2 with the 7 of a 3+1D
+ * one, 148 SMs); a second wave costs as much as the first.  Both forms give the
+ * same bits.  Measured, us per step fused / split, conformal: 101^2 (404
+ * blocks) 33 / 44, 129^2 (645) 56 / 51; table EoS: 101^2 42 / 54, 129^2
+ * 67 / 62, 25x25x11 (275) 45 / 59, 33x33x13 (858) 110 / 79, 41x37x21 205 / 89.
+ * Mixed: phase-split from 2^15 cells up (161^2 76 / 83, 201^2 102 / 93); its
+ * two forms round differently, so the line stays where its results have always
+ * changed form.  VH_STAGE_MODE=fused|split overrides. */
+static inline bool use_split(int nx, int ny, int nz, bool mixed)
 {
     static int forced = [] {
         const char *e = getenv("VH_STAGE_MODE");
         return !e ? -1 : (e[0] == 'f' ? 0 : 1);
     }();
     if (forced >= 0) return forced == 1;
-    return (long long)a.nx * a.ny * a.nz >= (1LL << 15);
+    if (mixed) return (long long)nx * ny * nz >= (1LL << 15);
+    return (long long)((nx + kFacesTX - 1) / kFacesTX) * ny * nz > 148 * (nz > 1 ? 2 : 3);
 }
 
 template <int NQ, int EOS, bool MIXED>
@@ -339,17 +351,25 @@ static void launch_stage_t(const StageArgs &a, cudaStream_t s, StageMarks *m)
         m->phase[m->n] = phase;
         cudaEventRecord(m->ev[++m->n], s);
     };
-    if (!use_split(a) && stage_faces()) {
+    const bool split = use_split(a.nx, a.ny, a.nz, MIXED);
+    if (!split && stage_faces()) {
         const dim3 gf((a.nx + kFacesTX - 1) / kFacesTX, a.ny, a.nz);
         const dim3 bf(kFacesTX, z ? 7 : 5, 1);
-        if (z && st2) kt_stage_faces_kernel<NQ, EOS, true, true, MIXED><<<gf, bf, 0, s>>>(a);
-        else if (z) kt_stage_faces_kernel<NQ, EOS, true, false, MIXED><<<gf, bf, 0, s>>>(a);
-        else if (st2) kt_stage_faces_kernel<NQ, EOS, false, true, MIXED><<<gf, bf, 0, s>>>(a);
-        else kt_stage_faces_kernel<NQ, EOS, false, false, MIXED><<<gf, bf, 0, s>>>(a);
+        /* dependent launch hides the FP64 kernel's launch; the mixed one is
+         * short, and waiting blocks take room from other events' kernels
+         * (three 101^2 events in turn: 206 -> 209 us per 10 steps) */
+        auto go = [&](auto kernel) {
+            if constexpr (MIXED) kernel<<<gf, bf, 0, s>>>(a);
+            else launch_pdl(kernel, gf, bf, 0, s, a);
+        };
+        if (z && st2) go(kt_stage_faces_kernel<NQ, EOS, true, true, MIXED>);
+        else if (z) go(kt_stage_faces_kernel<NQ, EOS, true, false, MIXED>);
+        else if (st2) go(kt_stage_faces_kernel<NQ, EOS, false, true, MIXED>);
+        else go(kt_stage_faces_kernel<NQ, EOS, false, false, MIXED>);
         mark(5);
         return;
     }
-    if (!use_split(a)) {
+    if (!split) {
         if (z && st2) kt_stage_kernel<NQ, EOS, true, true, MIXED><<<grid, block, 0, s>>>(a);
         else if (z) kt_stage_kernel<NQ, EOS, true, false, MIXED><<<grid, block, 0, s>>>(a);
         else if (st2) kt_stage_kernel<NQ, EOS, false, true, MIXED><<<grid, block, 0, s>>>(a);
