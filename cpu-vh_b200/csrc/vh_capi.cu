@@ -605,11 +605,8 @@ static void fo_args(vh_event *ev, vh::FoArgs &a)
     a.t0 = c.t0; a.dt = c.dt; a.t = ev->t; a.n = ev->n + 1;
     a.eos = dev_eos(ev);
     a.err.code = ev->err; a.err.step = ev->err + 1; a.err.cell = ev->err_cell;
-    /* scratch: [counts: ncubes+1][block sums][n_above][n_total] */
     a.counts = ev->fo_scratch;
-    a.block_sums = nullptr;
-    a.n_above = nullptr;
-    a.n_total = nullptr;
+    a.host_hdr = ev->fo_hdr;
     a.elems = ev->fo_elems;
     a.cap = ev->fo_cap;
     a.slots = ev->fo_slots;
@@ -628,6 +625,8 @@ int vh_event_freezeout_launch(vh_event *ev)
         CUDA_TRY(cudaMemsetAsync(ev->fo_slabs, 0, 2 * 11 * N * sizeof(double), ev->stream));
         ev->fo_scratch_ints = vh::freezeout_scratch_ints(c.nx, c.ny, c.nz);
         CUDA_TRY(ev_alloc(ev, &ev->fo_scratch, ev->fo_scratch_ints * sizeof(int)));
+        CUDA_TRY(cudaMemsetAsync(ev->fo_scratch + ev->fo_scratch_ints - vh::kFoHeaderInts, 0, vh::kFoHeaderInts * sizeof(int),
+                                 ev->stream));
         CUDA_TRY(cudaMallocHost(&ev->fo_hdr, 2 * sizeof(int)));
         CUDA_TRY(cudaEventCreateWithFlags(&ev->fo_done, cudaEventDisableTiming));
         /* a first element buffer sized for a surface crossing the lattice
@@ -650,9 +649,6 @@ int vh_event_freezeout_launch(vh_event *ev)
     fo_args(ev, a);
     vh::launch_freezeout(a, ev->stream);
     CUDA_TRY(cudaGetLastError());
-    /* header words 1 and 2: cells above e_F, elements */
-    CUDA_TRY(cudaMemcpyAsync(ev->fo_hdr, ev->fo_scratch + ev->fo_scratch_ints - vh::kFoHeaderInts + 1, 2 * sizeof(int),
-                             cudaMemcpyDeviceToHost, ev->stream));
     CUDA_TRY(cudaEventRecord(ev->fo_done, ev->stream));
     ev->fo_pending = true;
     return VH_OK;

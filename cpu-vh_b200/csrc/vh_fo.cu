@@ -3,24 +3,28 @@
  * swapAndSetHydroVariables + callFOFinder2p1D/3p1D + checkForCellsAboveTc
  * (freezeout/FreezeOut.cpp:57-381), which it runs serially over every cube.
  *
- * Pipeline (all on the event's stream):
- *   gather    current state -> coarse slab (11 planes over the interior) and
- *             the count of cells above e_F (warp-aggregated)
- *   classify  one thread per (hyper)cube between the previous and current
- *             slab: the above/below corner count; only cubes the surface
- *             crosses go on
- *   compact   exclusive scan of the flags -> dense list of crossed cubes, in
- *             the reference's loop order (ix outermost, then iy, then iz)
- *   count     Cornelius on each crossed cube -> number of elements
- *   scan      -> output offset of every cube's elements
- *   emit      Cornelius again, then the tri-/quadri-linear interpolation of
- *             the ten hydro fields at each centroid, T and P from the EoS,
- *             and the 20 surface.dat columns written at the cube's offset
+ * Pipeline (all on the event's stream, four kernels, each launched while the
+ * previous one drains):
+ *   open      current state -> coarse slab (11 planes over the interior), the
+ *             count of cells above e_F (warp-aggregated), and for every
+ *             (hyper)cube between the previous slab and the current state the
+ *             above/below corner count; cubes the surface crosses are
+ *             appended to a list, in no particular order
+ *   count     Cornelius on each listed cube -> its elements, kept in a slot,
+ *             and their number at the cube's index in the reference's loop
+ *             order (ix outermost, then iy, then iz)
+ *   offsets   exclusive scan of those numbers -> every cube's output offset
+ *   emit      the tri-/quadri-linear interpolation of the ten hydro fields
+ *             at each centroid, T and P from the EoS, and the 20 surface.dat
+ *             columns written at the cube's offset
  * The output is therefore in exactly the order the reference writes it.
- * Cubes crossed by the surface are a small fraction of the lattice, so
- * Cornelius runs twice on them rather than staging geometry in memory.
+ * Cubes crossed by the surface are a small fraction of the lattice.  (With a
+ * scan and a compaction of flags between gather, classification and count,
+ * the same block was thirteen launches: 62 us of device time on a 33x29
+ * event against 33.)
  */
 #include <cuda_runtime.h>
+#include <algorithm>
 #include "vh_kernels.h"
 #include "vh_cornelius.cuh"
 
@@ -34,68 +38,105 @@ static long long cube_count(int nx, int ny, int nz)
 
 size_t freezeout_scratch_ints(int nx, int ny, int nz)
 {
-    long long nc = cube_count(nx, ny, nz);
-    long long nb = (nc + 1 + kScanChunk - 1) / kScanChunk + 1;
-    /* flags/offsets, list, counts/offsets, block sums, header (n_straddle,
-     * n_above, n_total) */
-    return (size_t)((nc + 1) + nc + (nc + 1) + nb + kFoHeaderInts);
+    const long long nc = cube_count(nx, ny, nz), nb = (nc + 1 + kScanChunk - 1) / kScanChunk;
+    /* counts/offsets, list, chunk sums, header */
+    return (size_t)((nc + 1) + nc + nb + kFoHeaderInts);
 }
 
+/* hdr: [0] crossed cubes, [1] cells above e_F (both accumulated by the open
+ * step, zeroed again by the offsets step), [2] elements, [3] crossed cubes of
+ * the last block (for the emit step) */
 struct FoScratch {
-    int *flags, *list, *counts, *bsum, *hdr;   /* hdr: [0] crossed cubes, [1] cells above, [2] elements */
-    long long nc, nb;
+    int *counts, *list, *csum, *hdr;
+    int nc, nb;
 };
 
 static FoScratch carve(const FoArgs &a)
 {
     FoScratch s;
-    s.nc = cube_count(a.nx, a.ny, a.nz);
-    s.nb = (s.nc + 1 + kScanChunk - 1) / kScanChunk + 1;
-    s.flags = a.counts;
-    s.list = s.flags + s.nc + 1;
-    s.counts = s.list + s.nc;
-    s.bsum = s.counts + s.nc + 1;
-    s.hdr = s.bsum + s.nb;
+    s.nc = (int)cube_count(a.nx, a.ny, a.nz);        /* an event's padded cells number below 2^31 */
+    s.nb = (s.nc + 1 + kScanChunk - 1) / kScanChunk;
+    s.counts = a.counts;
+    s.list = s.counts + s.nc + 1;
+    s.csum = s.list + s.nc;
+    s.hdr = s.csum + s.nb;
     return s;
 }
 
-/* ------------------------------------------------------------ gather */
-__global__ void fo_gather_kernel(const __grid_constant__ FoArgs a, int *above)
+__device__ __forceinline__ void dep_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
+/* -------------------------------------------------------------- open */
+/* one thread per cell, x fastest: a warp's loads are contiguous.  It bounds
+ * itself by memory (11 planes read, 11 written, e of the previous slab). */
+__global__ void __launch_bounds__(256) fo_open_kernel(const __grid_constant__ FoArgs a, FoScratch sc)
 {
-    const long long N = (long long)a.nx * a.ny * a.nz;
-    const long long m = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    bool up = false;
+    dep_wait();       /* the state, and the scratch the previous block read */
+    dep_trigger();
+    const unsigned N = (unsigned)a.nx * a.ny * a.nz;
+    const unsigned m = blockIdx.x * blockDim.x + threadIdx.x;
+    bool up = false, cross = false;
+    int c = 0;
     if (m < N) {
-        const int ix = (int)(m % a.nx), iy = (int)((m / a.nx) % a.ny), iz = (int)(m / ((long long)a.nx * a.ny));
-        const long long L = a.L;
-        const long long s = (ix + 2) + (long long)a.ncx * ((iy + 2) + (long long)a.ncy * (iz + 2));
-        const double e = a.e[s];
-        double *c = a.slab_cur;
-        c[0 * N + m] = e;
-        c[1 * N + m] = a.u[1 * L + s];
-        c[2 * N + m] = a.u[2 * L + s];
-        c[3 * N + m] = a.u[3 * L + s];
-        c[4 * N + m] = e;
-        c[5 * N + m] = a.q[8 * L + s];
-        c[6 * N + m] = a.q[9 * L + s];
-        c[7 * N + m] = a.q[10 * L + s];
-        c[8 * N + m] = a.q[11 * L + s];
-        c[9 * N + m] = a.q[12 * L + s];
-        c[10 * N + m] = (a.nq == 15) ? a.q[14 * L + s] : 0.0;
-        up = e > a.eF;
+        const int r = m / a.nx, ix = m - r * a.nx, iz = r / a.ny, iy = r - iz * a.ny;
+        const long long L = a.L, sxy = (long long)a.ncx * a.ncy;
+        const long long s = (ix + 2) + (long long)a.ncx * (iy + 2) + sxy * (iz + 2);
+        const double *__restrict__ e = a.e + s;
+        const double e0 = e[0];
+        double *__restrict__ o = a.slab_cur + m;
+        const long long P = N;
+        o[0 * P] = e0;
+        o[1 * P] = a.u[1 * L + s];
+        o[2 * P] = a.u[2 * L + s];
+        o[3 * P] = a.u[3 * L + s];
+        o[4 * P] = e0;
+        o[5 * P] = a.q[8 * L + s];
+        o[6 * P] = a.q[9 * L + s];
+        o[7 * P] = a.q[10 * L + s];
+        o[8 * P] = a.q[11 * L + s];
+        o[9 * P] = a.q[12 * L + s];
+        o[10 * P] = (a.nq == 15) ? a.q[14 * L + s] : 0.0;
+        up = e0 > a.eF;
+        if ((int)m <= sc.nc) sc.counts[m] = 0;
+        if ((int)m < sc.nb) sc.csum[m] = 0;
+        const bool four = a.nz > 1;
+        if (ix < a.nx - 1 && iy < a.ny - 1 && (!four || iz < a.nz - 1)) {
+            const double *__restrict__ p = a.slab_prev + m;
+            int above = 0;
+#pragma unroll
+            for (int bz = 0; bz < 2; bz++) {
+                if (bz == 1 && !four) break;
+#pragma unroll
+                for (int by = 0; by < 2; by++)
+#pragma unroll
+                    for (int bx = 0; bx < 2; bx++) {
+                        above += e[bx + by * a.ncx + bz * sxy] >= a.eF;
+                        above += p[bx + by * a.nx + (long long)bz * a.nx * a.ny] >= a.eF;
+                    }
+            }
+            cross = above != 0 && above != (four ? 16 : 8);
+            c = iz + (four ? a.nz - 1 : 1) * (iy + (a.ny - 1) * ix);
+        }
     }
-    unsigned b = __ballot_sync(0xffffffffu, up);
-    if ((threadIdx.x & 31) == 0 && b) atomicAdd(above, __popc(b));
+    const unsigned b = __ballot_sync(0xffffffffu, up), x = __ballot_sync(0xffffffffu, cross);
+    const int lane = threadIdx.x & 31;
+    if (lane == 0 && b) atomicAdd(sc.hdr + 1, __popc(b));
+    if (x) {
+        int at = 0;
+        if (lane == 0) at = atomicAdd(sc.hdr, __popc(x));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (cross) sc.list[at + __popc(x & ((1u << lane) - 1))] = c;
+    }
 }
 
 /* cube index c enumerates (ix, iy, iz) with iz fastest, ix slowest: the
  * reference's loop nest order */
-__device__ __forceinline__ void cube_coords(const FoArgs &a, long long c, int &ix, int &iy, int &iz)
+__device__ __forceinline__ void cube_coords(const FoArgs &a, int c, int &ix, int &iy, int &iz)
 {
-    const int mz = a.nz > 1 ? a.nz - 1 : 1;
-    iz = (int)(c % mz);
-    iy = (int)((c / mz) % (a.ny - 1));
-    ix = (int)(c / ((long long)mz * (a.ny - 1)));
+    const int mz = a.nz > 1 ? a.nz - 1 : 1, r = c / mz;
+    iz = c - r * mz;
+    ix = r / (a.ny - 1);
+    iy = r - ix * (a.ny - 1);
 }
 
 __device__ __forceinline__ double slab(const FoArgs &a, int which, int v, int ix, int iy, int iz)
@@ -103,30 +144,6 @@ __device__ __forceinline__ double slab(const FoArgs &a, int which, int v, int ix
     const long long N = (long long)a.nx * a.ny * a.nz;
     const double *S = which ? a.slab_cur : a.slab_prev;
     return S[v * N + ix + (long long)a.nx * (iy + (long long)a.ny * iz)];
-}
-
-/* ----------------------------------------------------------- classify */
-/* threads run over the cubes in the slab's memory order (x fastest, so a
- * warp's corner loads are contiguous); each flag goes to the cube's index
- * in the reference's order (cube_coords) */
-__global__ void fo_classify_kernel(const __grid_constant__ FoArgs a, FoScratch sc)
-{
-    const long long m = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (m >= sc.nc) return;
-    const int mz = a.nz > 1 ? a.nz - 1 : 1;
-    const int ix = (int)(m % (a.nx - 1));
-    const int iy = (int)((m / (a.nx - 1)) % (a.ny - 1));
-    const int iz = (int)(m / ((long long)(a.nx - 1) * (a.ny - 1)));
-    const long long c = iz + (long long)mz * (iy + (long long)(a.ny - 1) * ix);
-    const bool four = a.nz > 1;
-    int above = 0;
-    for (int t = 0; t < 2; t++)
-        for (int bx = 0; bx < 2; bx++)
-            for (int by = 0; by < 2; by++)
-                for (int bz = 0; bz < (four ? 2 : 1); bz++)
-                    if (slab(a, t, 0, ix + bx, iy + by, iz + bz) >= a.eF) above++;
-    const int all = four ? 16 : 8;
-    sc.flags[c] = (above != 0 && above != all) ? 1 : 0;
 }
 
 /* -------------------------------------------------------------- scan */
@@ -213,11 +230,65 @@ void exclusive_scan(int *data, long long n, int *bsum, int *total, cudaStream_t 
     scan_apply_kernel<<<(unsigned)nb, kScanThreads, 0, st>>>(data, n, bsum, total);
 }
 
-__global__ void fo_compact_kernel(FoScratch sc)
+/* the output offset of every cube: each block scans one chunk of the counts
+ * from the sum of the chunks before it (at most a few hundred, added up by the
+ * block).  The last block writes the header, for the host too. */
+__global__ void __launch_bounds__(kScanThreads) fo_offsets_kernel(FoScratch sc, int *host_hdr)
 {
-    const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (c >= sc.nc) return;
-    if (sc.flags[c + 1] != sc.flags[c]) sc.list[sc.flags[c]] = (int)c;
+    __shared__ int red[33];
+    dep_wait();
+    dep_trigger();
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    int v = 0;
+    for (int k = tid; k < (int)blockIdx.x; k += kScanThreads) v += sc.csum[k];
+    const int i0 = blockIdx.x * kScanChunk + tid * kScanItems;
+    int loc[kScanItems], t = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+        loc[k] = (i0 + k < sc.nc) ? sc.counts[i0 + k] : 0;
+        t += loc[k];
+    }
+    /* block-wide: the sum of v and the inclusive scan of t */
+    int base = v, incl = t;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) base += __shfl_xor_sync(0xffffffffu, base, o);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+    }
+    __shared__ int tot[32];
+    if (lane == 31) tot[wid] = incl;
+    if (lane == 0) red[wid] = base;
+    __syncthreads();
+    if (wid == 0) {
+        int b = red[lane], w = tot[lane], ws = w;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, ws, o);
+            if (lane >= o) ws += u;
+        }
+        tot[lane] = ws - w;
+        if (lane == 0) red[32] = b;
+    }
+    __syncthreads();
+    int run = red[32] + tot[wid] + incl - t;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+        const int i = i0 + k;
+        if (i <= sc.nc) sc.counts[i] = run;
+        if (i == sc.nc) {
+            sc.hdr[2] = run;
+            sc.hdr[3] = sc.hdr[0];
+            host_hdr[0] = sc.hdr[1];
+            host_hdr[1] = run;
+            sc.hdr[0] = 0;
+            sc.hdr[1] = 0;
+        }
+        run += loc[k];
+    }
 }
 
 /* --------------------------------------------------------- Cornelius */
@@ -246,23 +317,35 @@ static_assert(cor::kMaxHedra <= cor::kMaxElements && cor::kMaxElements * 8 == kF
               "a cube's elements fit its slot");
 constexpr int kSlotDoubles = kFoSlotDoubles;
 
-__global__ void __launch_bounds__(128) fo_count_kernel(const __grid_constant__ FoArgs a, FoScratch sc)
+/* a listed cube's number of elements, at its place in the reference's order */
+__device__ __forceinline__ void put_count(const FoScratch &sc, int c, int ne)
 {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= sc.nc) return;
+    if (ne == 0) return;
+    sc.counts[c] = ne;
+    atomicAdd(sc.csum + c / kScanChunk, ne);
+}
+
+/* 2+1D: one thread per cube, one warp per block (the few hundred crossed cubes
+ * of an event spread over the SMs) */
+__global__ void __launch_bounds__(32) fo_count_kernel(const __grid_constant__ FoArgs a, FoScratch sc)
+{
+    dep_wait();
+    dep_trigger();
     const int nst = sc.hdr[0];
-    if (i >= nst) { sc.counts[i] = 0; return; }
-    int ix, iy, iz;
-    cube_coords(a, sc.list[i], ix, iy, iz);
-    cor::Work w;
-    double cen[cor::kMaxHedra][4], nor[cor::kMaxHedra][4];
-    int ne = cube_surface(a, ix, iy, iz, w, cen, nor);
-    if (ne < 0) { raise_error(a.err, 5, sc.list[i], a.n); ne = 0; }
-    sc.counts[i] = ne;
-    if (i < a.slot_cap) {
-        double *o = a.slots + i * kSlotDoubles;
-        for (int k = 0; k < ne; k++)
-            for (int d = 0; d < 4; d++) { o[8 * k + d] = cen[k][d]; o[8 * k + 4 + d] = nor[k][d]; }
+    for (int i = blockIdx.x * 32 + threadIdx.x; i < nst; i += gridDim.x * 32) {
+        const int c = sc.list[i];
+        int ix, iy, iz;
+        cube_coords(a, c, ix, iy, iz);
+        cor::Work w;
+        double cen[cor::kMaxHedra][4], nor[cor::kMaxHedra][4];
+        int ne = cube_surface(a, ix, iy, iz, w, cen, nor);
+        if (ne < 0) { raise_error(a.err, 5, c, a.n); ne = 0; }
+        put_count(sc, c, ne);
+        if (i < a.slot_cap) {
+            double *o = a.slots + (long long)i * kSlotDoubles;
+            for (int k = 0; k < ne; k++)
+                for (int d = 0; d < 4; d++) { o[8 * k + d] = cen[k][d]; o[8 * k + 4 + d] = nor[k][d]; }
+        }
     }
 }
 
@@ -386,10 +469,9 @@ __global__ void __launch_bounds__(128, 3) fo_count4_kernel(const __grid_constant
     Count4Shared &S = *reinterpret_cast<Count4Shared *>(count4_smem);
     const int tid = threadIdx.x, g = tid >> 3, q = tid & 7, lane = tid & 31, wid = tid >> 5;
     const unsigned gmask = 0xFFu << (lane & ~7);
+    dep_wait();
+    dep_trigger();
     const int nst = sc.hdr[0];
-    /* the uncrossed entries of the counts the offsets are scanned from */
-    for (long long i = nst + (long long)blockIdx.x * 128 + tid; i < sc.nc; i += (long long)gridDim.x * 128)
-        sc.counts[i] = 0;
     const double dx[4] = {a.dtau_c, a.dx, a.dy, a.dz};
     const double E0 = a.eF;
     const cor::WorkRef pool{S.p, S.out, S.flip, S.poly, 0, 0, kPoolLines, kPoolPolys, false};
@@ -538,7 +620,7 @@ __global__ void __launch_bounds__(128, 3) fo_count4_kernel(const __grid_constant
                 if (q == 0) {
                     int ne = nh;
                     if (ne < 0) { raise_error(a.err, 5, sc.list[hidx], a.n); ne = 0; }
-                    sc.counts[hidx] = ne;
+                    put_count(sc, sc.list[hidx], ne);
                 }
                 done = true;
             } else if (!done && q == 0) {
@@ -554,6 +636,22 @@ __global__ void __launch_bounds__(128, 3) fo_count4_kernel(const __grid_constant
     }
 }
 
+template <typename... P, typename... X>
+static void launch_dep(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, const X &...x)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, x...);
+}
+
 static void launch_count4(const FoArgs &a, FoScratch sc, cudaStream_t st)
 {
     static int blocks = [] {
@@ -565,9 +663,9 @@ static void launch_count4(const FoArgs &a, FoScratch sc, cudaStream_t st)
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fo_count4_kernel, 128, sizeof(Count4Shared));
         return sms * (per_sm > 0 ? per_sm : 1);
     }();
-    const long long need = (sc.nc + kG4 - 1) / kG4;
+    const long long need = ((long long)sc.nc + kG4 - 1) / kG4;
     const unsigned grid = (unsigned)(need < blocks ? (need > 0 ? need : 1) : blocks);
-    fo_count4_kernel<<<grid, 128, sizeof(Count4Shared), st>>>(a, sc);
+    launch_dep(fo_count4_kernel, grid, 128, sizeof(Count4Shared), st, a, sc);
 }
 
 /* FreezeOut.cpp:40-55 */
@@ -646,44 +744,92 @@ static __device__ __noinline__ void emit_recompute(const FoArgs &a, int ix, int 
     }
 }
 
+/* emit_element spread over sixteen lanes: one field each (0-9; lane 3, which
+ * holds e, also T and P), one coordinate of position and normal each (10-13) */
 template <int EOS>
-__global__ void __launch_bounds__(128) fo_emit_kernel(const __grid_constant__ FoArgs a, FoScratch sc)
+__device__ __forceinline__ void emit_lane(const FoArgs &a, int ix, int iy, int iz, const double *cen, const double *nor,
+                                          double *__restrict__ o, int lane)
 {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= sc.nc || i >= sc.hdr[0]) return;
-    int ix, iy, iz;
-    cube_coords(a, sc.list[i], ix, iy, iz);
-    const long long off = sc.counts[i];
-    if (i >= a.slot_cap) { emit_recompute<EOS>(a, ix, iy, iz, off); return; }
-    const int ne = sc.counts[i + 1] - sc.counts[i];
-    const double *sl = a.slots + i * kSlotDoubles;
-    for (int k = 0; k < ne; k++) {
-        if (off + k >= a.cap) return;
-        emit_element<EOS>(a, ix, iy, iz, sl + 8 * k, sl + 8 * k + 4, a.elems + (off + k) * VH_FO_COLUMNS);
+    const bool four = a.nz > 1;
+    if (lane < 10) {
+        const int v = lane;
+        double f;
+        if (four) {
+            const double tf = cen[0] / a.dtau_c, xf = cen[1] / a.dx, yf = cen[2] / a.dy, zf = cen[3] / a.dz;
+            double c[16];
+#pragma unroll
+            for (int t = 0; t < 2; t++)
+#pragma unroll
+                for (int bx = 0; bx < 2; bx++)
+#pragma unroll
+                    for (int by = 0; by < 2; by++)
+#pragma unroll
+                        for (int bz = 0; bz < 2; bz++)
+                            c[t * 8 + bx * 4 + by * 2 + bz] = slab(a, t, v + 1, ix + bx, iy + by, iz + bz);
+            f = interp4(tf, xf, yf, zf, c);
+        } else {
+            const double tf = cen[1] / a.dtau_c, xf = cen[2] / a.dx, yf = cen[3] / a.dy;
+            f = interp3(tf, xf, yf, slab(a, 0, v + 1, ix, iy, 0), slab(a, 1, v + 1, ix, iy, 0),
+                        slab(a, 0, v + 1, ix + 1, iy, 0), slab(a, 0, v + 1, ix, iy + 1, 0),
+                        slab(a, 1, v + 1, ix + 1, iy, 0), slab(a, 1, v + 1, ix, iy + 1, 0),
+                        slab(a, 0, v + 1, ix + 1, iy + 1, 0), slab(a, 1, v + 1, ix + 1, iy + 1, 0));
+        }
+        o[v < 4 ? 8 + v : 10 + v] = f;
+        if (v == 3) {
+            o[12] = eos_T<EOS>(a.eos, f);
+            o[13] = eos_p<EOS>(a.eos, f);
+        }
+    } else if (lane < 14) {
+        const int d = lane - 10, n = (d == 0) ? 0 : (d == 1) ? a.nx : (d == 2) ? a.ny : a.nz;
+        const int i = (d == 1) ? ix : (d == 2) ? iy : iz;
+        const double h = (d == 1) ? a.dx : (d == 2) ? a.dy : a.dz;
+        const double cell = (d == 0) ? a.t0 + ((double)a.n) * a.dt : (double)i * h - (((double)(n - 1)) / 2.0 * h);
+        if (four) {
+            o[d] = cen[d] + cell;
+            o[4 + d] = a.t * nor[d];
+        } else {
+            o[d] = (d < 3) ? cen[d + 1] + cell : 0.0;
+            o[4 + d] = (d < 3) ? a.t * nor[d + 1] : 0.0;
+        }
     }
 }
 
-__global__ void fo_header_kernel(FoScratch sc)
+/* sixteen lanes per crossed cube: one thread per cube leaves its 160 scattered
+ * corner loads per element to a few warps (19.5 -> 8 us per block of a
+ * 41x37x21 event). */
+template <int EOS>
+__global__ void __launch_bounds__(128) fo_emit_kernel(const __grid_constant__ FoArgs a, FoScratch sc)
 {
-    /* hdr[0] = number of crossed cubes (flags scanned in place: flags[nc]) */
-    sc.hdr[0] = sc.flags[sc.nc];
+    dep_wait();
+    dep_trigger();
+    const int nst = sc.hdr[3], lane = threadIdx.x & 15, kept = min(nst, a.slot_cap);
+    for (int i = blockIdx.x * 8 + (threadIdx.x >> 4); i < kept; i += gridDim.x * 8) {
+        const int c = sc.list[i];
+        int ix, iy, iz;
+        cube_coords(a, c, ix, iy, iz);
+        const long long off = sc.counts[c];
+        const int ne = sc.counts[c + 1] - (int)off;
+        const double *sl = a.slots + (long long)i * kSlotDoubles;
+        for (int k = 0; k < ne && off + k < a.cap; k++)
+            emit_lane<EOS>(a, ix, iy, iz, sl + 8 * k, sl + 8 * k + 4, a.elems + (off + k) * VH_FO_COLUMNS, lane);
+    }
+    /* cubes beyond the slots: a thread each */
+    for (int i = kept + blockIdx.x * 128 + threadIdx.x; i < nst; i += gridDim.x * 128) {
+        const int c = sc.list[i];
+        int ix, iy, iz;
+        cube_coords(a, c, ix, iy, iz);
+        emit_recompute<EOS>(a, ix, iy, iz, sc.counts[c]);
+    }
 }
 
 void launch_freezeout(const FoArgs &a, cudaStream_t st)
 {
-    FoScratch sc = carve(a);
-    const long long N = (long long)a.nx * a.ny * a.nz;
-    cudaMemsetAsync(sc.hdr, 0, kFoHeaderInts * sizeof(int), st);
-    fo_gather_kernel<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(a, sc.hdr + 1);
-    const unsigned gc = (unsigned)((sc.nc + 255) / 256);
-    fo_classify_kernel<<<gc, 256, 0, st>>>(a, sc);
-    exclusive_scan(sc.flags, sc.nc, sc.bsum, nullptr, st);
-    fo_compact_kernel<<<gc, 256, 0, st>>>(sc);
-    fo_header_kernel<<<1, 1, 0, st>>>(sc);
-    const unsigned gk = (unsigned)((sc.nc + 127) / 128);
+    const FoScratch sc = carve(a);
+    const unsigned N = (unsigned)a.nx * a.ny * a.nz;
+    launch_dep(fo_open_kernel, (N + 255) / 256, 256, 0, st, a, sc);
     if (a.nz > 1) launch_count4(a, sc, st);
-    else fo_count_kernel<<<gk, 128, 0, st>>>(a, sc);
-    exclusive_scan(sc.counts, sc.nc, sc.bsum, sc.hdr + 2, st);
+    else launch_dep(fo_count_kernel, (unsigned)std::min((sc.nc + 31) / 32, 148 * 16), 32, 0, st, a, sc);
+    launch_dep(fo_offsets_kernel, (unsigned)sc.nb, kScanThreads, 0, st, sc, a.host_hdr);
     launch_freezeout_emit(a, st);
 }
 
@@ -692,10 +838,10 @@ void launch_freezeout(const FoArgs &a, cudaStream_t st)
 void launch_freezeout_emit(const FoArgs &a, cudaStream_t st)
 {
     if (!a.elems || a.cap <= 0) return;
-    FoScratch sc = carve(a);
-    const unsigned gk = (unsigned)((sc.nc + 127) / 128);
-    if (a.eos.kind == 1) fo_emit_kernel<1><<<gk, 128, 0, st>>>(a, sc);
-    else fo_emit_kernel<0><<<gk, 128, 0, st>>>(a, sc);
+    const FoScratch sc = carve(a);
+    const unsigned grid = (unsigned)std::min((sc.nc + 7) / 8, 148 * 16);
+    if (a.eos.kind == 1) launch_dep(fo_emit_kernel<1>, grid, 128, 0, st, a, sc);
+    else launch_dep(fo_emit_kernel<0>, grid, 128, 0, st, a, sc);
 }
 
 } // namespace vh

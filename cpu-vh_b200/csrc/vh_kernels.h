@@ -139,25 +139,22 @@ struct FoArgs {
     int n;                       /* loop index of the freezeout block */
     DevEos eos;
     DevErr err;
-    int *counts;                 /* per (hyper)cube element counts, then offsets */
-    int *block_sums;
-    int *n_above;                /* cells above eF */
+    int *counts;                 /* scratch (freezeout_scratch_ints): per (hyper)cube element counts, then offsets, ... */
+    int *host_hdr;               /* pinned: cells above eF, elements */
     double *elems;               /* output, VH_FO_COLUMNS per element */
     int cap;                     /* capacity of elems in elements */
     double *slots;               /* centroids and normals of the first slot_cap crossed cubes */
     int slot_cap;
-    int *n_total;
 };
 
 /* doubles of one crossed cube's element slot: up to 10 elements (Cornelius
  * MAX_ELEMENTS), centroid and normal (4 + 4) each */
 constexpr int kFoSlotDoubles = 80;
-/* the freezeout scratch ends with its header: crossed cubes, cells above
- * e_F, elements */
-constexpr int kFoHeaderInts = 3;
+/* the freezeout scratch ends with its header, zero before the first block */
+constexpr int kFoHeaderInts = 4;
 
-/* Runs the whole freezeout block; returns the number of elements through
- * *a.n_total (device) and leaves elements in a.elems. */
+/* Runs the whole freezeout block; leaves the elements in a.elems and the
+ * cells above e_F and the number of elements in a.host_hdr. */
 void launch_freezeout(const FoArgs &a, cudaStream_t s);
 /* nz = 1: write the eta ghost planes of one padded field plane (ncz = 5) */
 void launch_eta_ghost_fill(double *plane, int nx, int ny, int ncx, int ncy, cudaStream_t s);
