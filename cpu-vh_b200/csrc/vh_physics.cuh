@@ -283,6 +283,7 @@ __device__ __forceinline__ Prim infer(const DevEos &E, double t, double M0, doub
  * ------------------------------------------------------------------ */
 struct Flow { double ut, v, y; };       /* u^tau, u^dir, RN(1/u^tau) */
 
+template <bool MIXED = false>
 __device__ __forceinline__ double eos_interp_direct(const DevEos &E, double ed, const double *tb)
 {
     /* ed - e_min and ed minus a node are 0 or far above 2^-900 for ed >=
@@ -291,12 +292,24 @@ __device__ __forceinline__ double eos_interp_direct(const DevEos &E, double ed, 
     idx = (E.e_length - 2 < idx) ? E.e_length - 2 : idx;
     idx = (idx < 0) ? 0 : idx;
     const double frac = div_rn(ed - (idx * E.e_spacing + E.e_min), E.e_spacing, E.inv_spacing);
-    return __ldg(tb + idx) * (1. - frac) + __ldg(tb + idx + 1) * frac;
+    const double lo = __ldg(tb + idx), hi = __ldg(tb + idx + 1);
+    /* the mixed translation unit contracts eos_interp's sum this way */
+    if (MIXED) return fma(lo, 1. - frac, hi * frac);
+    return lo * (1. - frac) + hi * frac;
+}
+
+/* the FP32 square root as infer takes it: correctly rounded, or in the mixed
+ * translation unit the fast one its sqrtf compiles to (branch-free anyway) */
+template <bool MIXED>
+__device__ __forceinline__ float root32(float x)
+{
+    if constexpr (MIXED) return sqrtf(x);
+    else return sqrt_rn(x);
 }
 
 /* the energy density of N states (e_from_conserved, or infer's closed form
  * below ePrev = 0.1); M = M1^2 + M2^2 + t^2 M3^2 */
-template <int EOS, int N>
+template <int EOS, int N, bool MIXED>
 __device__ __forceinline__ bool energy_direct(const DevEos &E, const double (&M0)[N], const double (&M)[N],
                                               const double (&Pi)[N], double ePrev, double (&ef)[N])
 {
@@ -314,7 +327,7 @@ __device__ __forceinline__ bool energy_direct(const DevEos &E, const double (&M0
         for (int s = 0; s < N; ++s) {
             const float h2 = fabsf(__double2float_rn(4 * M0[s] * M0[s] - 3 * M[s]));
             ok = ok && in_range(h2);
-            ef[s] = (double)fabsf(__double2float_rn((double)sqrt_rn(h2) - M0[s]));
+            ef[s] = (double)fabsf(__double2float_rn((double)root32<MIXED>(h2) - M0[s]));
         }
     } else {
         double e0[N], B[N];
@@ -333,14 +346,14 @@ __device__ __forceinline__ bool energy_direct(const DevEos &E, const double (&M0
             for (int s = 0; s < N; ++s) {
                 const double x = e0[s];
                 bool fine = (unsigned)__double2hiint(x) - ((1023u - 60u) << 20) < E.direct && rcp_ok(x);
-                const double pp = eos_interp_direct(E, x, E.p_tb);     /* above the floor */
+                const double pp = eos_interp_direct<MIXED>(E, x, E.p_tb);     /* above the floor */
                 fine = fine && within<-49, 60>(pp);
                 const double yx = rcp_rn(x);
                 const double cst2 = div_rn(pp, x, yx);
                 const double A = M0[s] * (1.0 - cst2) + Pi[s];
                 const float h2 = fabsf(__double2float_rn(A * A + 4 * cst2 * B[s]));
                 fine = fine && in_range(h2);
-                const double H = (double)sqrt_rn(h2);
+                const double H = (double)root32<MIXED>(h2);
                 const double c2 = 2 * cst2;
                 const double D = div_rn(A - H, c2, rcp_rn(c2));
                 const double f = x + D;
@@ -369,25 +382,25 @@ __device__ __forceinline__ bool energy_direct(const DevEos &E, const double (&M0
 
 /* infer's e, p (floored), u^tau, RN(1/u^tau) and 1/((e + P) u^tau) from the
  * energy density; the last times M1..M3 is the velocity while u^tau <= 1e3 */
-template <int EOS>
+template <int EOS, bool MIXED>
 __device__ __forceinline__ bool flow_direct(const DevEos &E, double M0, double Pi, double &e, double &p, double &ut,
                                             double &yu, double &E2)
 {
     const bool low = e < 1.e-7;
     bool ok = low || in_range(e);
-    p = (EOS == 1) ? floor15(eos_interp_direct(E, e, E.p_tb)) : div_rn(e, 3., 1. / 3.);
+    p = (EOS == 1) ? floor15(eos_interp_direct<MIXED>(E, e, E.p_tb)) : div_rn(e, 3., 1. / 3.);
     if (low) { e = 1.e-7; p = 1.e-7; }
     const double P = p + Pi, W = e + P;
     const double Einv = rcp_rn(W);
     const float x = fabsf(__double2float_rn((M0 + P) * Einv));
     ok = ok && in_range_abs(W) && rcp_ok(W) && in_range(x);
-    ut = (double)sqrt_rn(x);          /* 24 significant bits: rcp_ok */
+    ut = (double)root32<MIXED>(x);          /* 24 significant bits: rcp_ok */
     yu = rcp_rn(ut);
     E2 = div_rn(Einv, ut, yu);
     return ok;
 }
 
-template <int EOS>
+template <int EOS, bool MIXED = false>
 __device__ __forceinline__ bool flow_pair(const DevEos &E, double t, const double (&M0)[2], const double (&M1)[2],
                                           const double (&M2)[2], const double (&M3)[2], const double (&Pi)[2], int dir,
                                           double ePrev, Flow (&out)[2])
@@ -395,11 +408,11 @@ __device__ __forceinline__ bool flow_pair(const DevEos &E, double t, const doubl
     double M[2], ef[2];
 #pragma unroll
     for (int s = 0; s < 2; ++s) M[s] = M1[s] * M1[s] + M2[s] * M2[s] + t * t * M3[s] * M3[s];
-    bool ok = energy_direct<EOS, 2>(E, M0, M, Pi, ePrev, ef);
+    bool ok = energy_direct<EOS, 2, MIXED>(E, M0, M, Pi, ePrev, ef);
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
         double p, ut, yu, E2;
-        ok = flow_direct<EOS>(E, M0[s], Pi[s], ef[s], p, ut, yu, E2) && ok;
+        ok = flow_direct<EOS, MIXED>(E, M0[s], Pi[s], ef[s], p, ut, yu, E2) && ok;
         double v = ((dir == 1) ? M1[s] : (dir == 2) ? M2[s] : M3[s]) * E2;
         if (ut > 1.0e3) { ut = 1.0; v = 0.0; yu = 1.0; }
         out[s].ut = ut;
@@ -416,9 +429,9 @@ __device__ __forceinline__ bool infer_direct(const DevEos &E, double t, double M
 {
     const double M0s[1] = {M0}, M[1] = {M1 * M1 + M2 * M2 + t * t * M3 * M3}, Pis[1] = {Pi};
     double ef[1], yu, E2;
-    bool ok = energy_direct<EOS, 1>(E, M0s, M, Pis, ePrev, ef);
+    bool ok = energy_direct<EOS, 1, false>(E, M0s, M, Pis, ePrev, ef);
     r.e = ef[0];
-    ok = flow_direct<EOS>(E, M0, Pi, r.e, r.p, r.ut, yu, E2) && ok;
+    ok = flow_direct<EOS, false>(E, M0, Pi, r.e, r.p, r.ut, yu, E2) && ok;
     r.ux = M1 * E2;
     r.uy = M2 * E2;
     r.un = M3 * E2;

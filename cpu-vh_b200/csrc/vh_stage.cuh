@@ -995,8 +995,12 @@ __device__ __forceinline__ void extrapolate_m(const double *__restrict__ qn, lon
     qL = B + (double)(0.5f * slope_f(th, A, B, C));
 }
 
-/* face_flux with FP32 slopes and flux arithmetic; FP64 half-site states and root solve */
-template <int NQ, int EOS>
+/* face_flux with FP32 slopes and flux arithmetic; FP64 half-site states and
+ * root solve (flow_pair).  The fused multiply-adds of the flux are written out,
+ * so that its rounding does not hang on how the compiler contracts the sum in
+ * one kernel or another; LFIRST: sL qL is the product that is added unrounded
+ * (the face a cell evaluates for itself across the e <= 0.1 branch). */
+template <int NQ, int EOS, bool LFIRST = false>
 __device__ __forceinline__ void face_flux_m(const StageArgs &A, long long b, long long st, int dir, bool fwd,
                                             double ePrev, double *__restrict__ r, bool &bad)
 {
@@ -1008,11 +1012,20 @@ __device__ __forceinline__ void face_flux_m(const StageArgs &A, long long b, lon
     for (int c = 0; c < 8; ++c) extrapolate_m(q + c * L, b, st, th, qRs[c], qLs[c]);
     double PiR = 0, PiL = 0;
     if (NQ == 15) extrapolate_m(q + 14 * L, b, st, th, PiR, PiL);
-    Prim R = infer<EOS, true>(A.eos, A.t, qRs[0] - qRs[4], qRs[1] - qRs[5], qRs[2] - qRs[6], qRs[3] - qRs[7], PiR, ePrev, bad);
-    Prim Lf = infer<EOS, true>(A.eos, A.t, qLs[0] - qLs[4], qLs[1] - qLs[5], qLs[2] - qLs[6], qLs[3] - qLs[7], PiL, ePrev, bad);
-    const float vR = (float)((dir == 1) ? R.ux : (dir == 2) ? R.uy : R.un);
-    const float vL = (float)((dir == 1) ? Lf.ux : (dir == 2) ? Lf.uy : Lf.un);
-    const float sR = vR / (float)R.ut, sL = vL / (float)Lf.ut;
+    const double M0[2] = {qRs[0] - qRs[4], qLs[0] - qLs[4]}, M1[2] = {qRs[1] - qRs[5], qLs[1] - qLs[5]};
+    const double M2[2] = {qRs[2] - qRs[6], qLs[2] - qLs[6]}, M3[2] = {qRs[3] - qRs[7], qLs[3] - qLs[7]};
+    const double Pi[2] = {PiR, PiL};
+    bool direct = A.eos.direct != 0 && half_state_ranged(PiR) && half_state_ranged(PiL);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) direct = direct && half_state_ranged(qRs[c]) && half_state_ranged(qLs[c]);
+    Flow F[2];
+    direct = flow_pair<EOS, true>(A.eos, A.t, M0, M1, M2, M3, Pi, dir, ePrev, F) && direct;
+    float sR = (float)F[0].v / (float)F[0].ut, sL = (float)F[1].v / (float)F[1].ut;
+    if (!direct) {
+        flow_pair_plain<EOS>(A.eos, A.t, M0, M1, M2, M3, Pi, dir, ePrev, F, bad);
+        sR = (float)F[0].v / (float)F[0].ut;
+        sL = (float)F[1].v / (float)F[1].ut;
+    }
     const float a = fmaxf(fabsf(sL), fabsf(sR));
 #pragma unroll
     for (int n = 0; n < NQ; ++n) {
@@ -1020,7 +1033,8 @@ __device__ __forceinline__ void face_flux_m(const StageArgs &A, long long b, lon
         if (n < 8) { qR = qRs[n]; qL = qLs[n]; }
         else if (n == 14) { qR = PiR; qL = PiL; }
         else extrapolate_m(q + n * L, b, st, th, qR, qL);
-        const float res = 0.5f * (sR * (float)qR + sL * (float)qL - a * (float)(qR - qL));
+        const float fR = (float)qR, fL = (float)qL;
+        const float res = 0.5f * fmaf(-a, (float)(qR - qL), LFIRST ? fmaf(sL, fL, sR * fR) : fmaf(sR, fR, sL * fL));
         r[n] = fwd ? -(double)res : r[n] + (double)res;
     }
 }
@@ -1157,13 +1171,13 @@ __device__ __forceinline__ void stage_body_m(const StageArgs &A, int i, int j, i
  * y (eta) the block's second index runs along y (eta) and the last row of
  * threads only computes faces.
  * --------------------------------------------------------------------- */
-template <int NQ, int EOS>
+template <int NQ, int EOS, bool LFIRST = false>
 __device__ __forceinline__ void face_H_m(const StageArgs &A, long long b, long long st, int dir, double ePrev,
                                          double *__restrict__ H, bool &bad)
 {
 #pragma unroll
     for (int n = 0; n < NQ; ++n) H[n] = 0.0;
-    face_flux_m<NQ, EOS>(A, b, st, dir, false, ePrev, H, bad);
+    face_flux_m<NQ, EOS, LFIRST>(A, b, st, dir, false, ePrev, H, bad);
 }
 
 /* one tile of the face-once flux along DIR; (i0, j0, k0) interior coordinates
@@ -1220,7 +1234,7 @@ __device__ __forceinline__ void flux_faces_tile(const StageArgs &A, int i0, int 
         const double e_self = __ldg(A.ein + s), e_next = __ldg(A.ein + s + st);
         if ((e_self <= 0.1) != (e_next <= 0.1)) {
             double F[NQ];
-            face_H_m<NQ, EOS>(A, s, st, DIR, e_self, F, bad);
+            face_H_m<NQ, EOS, true>(A, s, st, DIR, e_self, F, bad);
 #pragma unroll
             for (int n = 0; n < NQ; ++n) r[n] = H[n] - F[n];
         } else {
@@ -1297,31 +1311,39 @@ __device__ __forceinline__ void flux_faces_lines(const StageArgs &A, double *__r
     }
 #pragma unroll
     for (int n = 0; n < NQ; ++n) sm[n * 128 + tid] = H[n];
+    const bool update = face_ok && f < nd && pr < PB - 1;
+    const double d = (DIR == 1) ? A.dx : (DIR == 2) ? A.dy : A.dz;
+    const double yd = (DIR == 1) ? A.inv_dx : (DIR == 2) ? A.inv_dy : A.inv_dz;
+    /* what the update reads, requested before the barrier: the wait for the
+     * neighbour's face covers it */
+    double S[4], e_self = 0, e_next = 0, acc[NQ];
+    if (PDL) pdl_wait();
+    if (update) {
+#pragma unroll
+        for (int n = 0; n < NQ; ++n) acc[n] = A.qout[n * A.L + s];
+        e_self = __ldg(A.ein + s);
+        e_next = __ldg(A.ein + s + st);
+        dir_sources<NQ>(A, s, st, d, DIR, S);
+    }
     __syncthreads();
-    if (face_ok && f < nd && pr < PB - 1) {
+    if (update) {
         const int nxt = tid + W;                  /* face f + 1 of the same line */
-        const double d = (DIR == 1) ? A.dx : (DIR == 2) ? A.dy : A.dz;
-        const double yd = (DIR == 1) ? A.inv_dx : (DIR == 2) ? A.inv_dy : A.inv_dz;
         double r[NQ];
-        const double e_self = __ldg(A.ein + s), e_next = __ldg(A.ein + s + st);
         if ((e_self <= 0.1) != (e_next <= 0.1)) {
             double F[NQ];
-            face_H_m<NQ, EOS>(A, s, st, DIR, e_self, F, bad);
+            face_H_m<NQ, EOS, true>(A, s, st, DIR, e_self, F, bad);
 #pragma unroll
             for (int n = 0; n < NQ; ++n) r[n] = H[n] - F[n];
         } else {
 #pragma unroll
             for (int n = 0; n < NQ; ++n) r[n] = H[n] - sm[n * 128 + nxt];
         }
-        double S[4];
-        dir_sources<NQ>(A, s, st, d, DIR, S);
 #pragma unroll
         for (int n = 0; n < 4; ++n) r[n] = (r[n] * yd + S[n]) * A.dt;
 #pragma unroll
         for (int n = 4; n < NQ; ++n) r[n] *= yd * A.dt;
-        if (PDL) pdl_wait();
 #pragma unroll
-        for (int n = 0; n < NQ; ++n) A.qout[n * A.L + s] += r[n];
+        for (int n = 0; n < NQ; ++n) A.qout[n * A.L + s] = acc[n] + r[n];
     }
     if (bad) raise_error(A.err, kErrNan, s, A.step);
 }
