@@ -144,9 +144,10 @@ long long batch_line_blocks(int dir, int nx, int ny, int nz)
 
 long long batch_face_line_blocks(int dir, int nx, int ny, int nz)
 {
-    const int nd = dir == 2 ? ny : nz;
-    const long long bund = dir == 2 ? FaceLinesG<2>::bundles(nx, ny, nz) : FaceLinesG<3>::bundles(nx, ny, nz);
-    const int pb = dir == 2 ? FaceLinesG<2>::PB : FaceLinesG<3>::PB;
+    const int nd = dir == 1 ? nx : dir == 2 ? ny : nz;
+    const long long bund = dir == 1 ? FaceLinesG<1>::bundles(nx, ny, nz) : dir == 2 ? FaceLinesG<2>::bundles(nx, ny, nz)
+                                                                          : FaceLinesG<3>::bundles(nx, ny, nz);
+    const int pb = dir == 1 ? FaceLinesG<1>::PB : dir == 2 ? FaceLinesG<2>::PB : FaceLinesG<3>::PB;
     return ((long long)(nd + 1) * bund + pb - 2) / (pb - 1);
 }
 
@@ -205,7 +206,7 @@ struct vh_batch {
     std::map<int, Tiles> tiles;      /* key: tile_x */
     int4 *ftiles[3] = {};            /* mixed precision: face tiles per axis */
     int n_ftiles[3] = {};
-    int4 *fltiles[3] = {};           /* mixed precision: face line blocks along y, eta */
+    int4 *fltiles[3] = {};           /* mixed precision: face line blocks per axis */
     int n_fltiles[3] = {};
     int4 *ltiles[3] = {};            /* FP64: line blocks (member, block) per axis */
     int n_ltiles[3] = {};
@@ -285,16 +286,16 @@ int build_face_tiles(vh_batch *b)
         BTRY(cudaMalloc(&b->ftiles[d], f[d].size() * sizeof(int4)));
         BTRY(cudaMemcpy(b->ftiles[d], f[d].data(), f[d].size() * sizeof(int4), cudaMemcpyHostToDevice));
     }
-    /* face line blocks along y and eta (the 3+1D members) */
+    /* face line blocks (along eta: the 3+1D members) */
     std::vector<int4> fl[3];
     for (size_t m = 0; m < b->mem.size(); ++m) {
         const vh_config &c = b->mem[m]->cfg;
-        for (int d = 2; d <= (c.nz > 1 ? 3 : 2); ++d) {
+        for (int d = 1; d <= (c.nz > 1 ? 3 : 2); ++d) {
             const long long nb = vh::batch_face_line_blocks(d, c.nx, c.ny, c.nz);
             for (long long k = 0; k < nb; ++k) fl[d - 1].push_back(make_int4((int)m, (int)k, 0, 0));
         }
     }
-    for (int d = 1; d < 3; ++d) {
+    for (int d = 0; d < 3; ++d) {
         b->n_fltiles[d] = (int)fl[d].size();
         if (fl[d].empty()) continue;
         BTRY(cudaMalloc(&b->fltiles[d], fl[d].size() * sizeof(int4)));
@@ -303,7 +304,7 @@ int build_face_tiles(vh_batch *b)
     return VH_OK;
 }
 
-/* mixed batches run their y and eta flux over face line pieces (the
+/* mixed batches run their flux over face line pieces (the
  * single-event form); VH_BATCH_FACE_LINES=0 keeps the 32 x 8 face tiles */
 bool batch_face_lines_on()
 {
@@ -448,7 +449,7 @@ void launch_face(vh_batch *b, int stage, int dir)
 {
     vh::BatchLaunch B;
     B.args = b->d_args + (size_t)stage * b->mem.size();
-    if (dir >= 2 && batch_face_lines_on()) {
+    if (batch_face_lines_on()) {
         B.tiles = b->fltiles[dir - 1];
         B.ntiles = b->n_fltiles[dir - 1];
         if (B.ntiles == 0) return;
@@ -627,7 +628,7 @@ int preload(vh_batch *b)
         }
     if (b->mixed) {
         for (int d = 1; d <= 3; ++d) BTRY(cudaFuncGetAttributes(&attr, vh::batch_face_kernel_mixed(b->nq, b->eos_kind, d)));
-        for (int d = 2; d <= 3; ++d) BTRY(cudaFuncGetAttributes(&attr, vh::batch_face_lines_kernel_mixed(b->nq, b->eos_kind, d)));
+        for (int d = 1; d <= 3; ++d) BTRY(cudaFuncGetAttributes(&attr, vh::batch_face_lines_kernel_mixed(b->nq, b->eos_kind, d)));
     }
     else
         for (int d = 1; d <= 3; ++d) BTRY(cudaFuncGetAttributes(&attr, vh::batch_lines_kernel(b->nq, b->eos_kind, d)));

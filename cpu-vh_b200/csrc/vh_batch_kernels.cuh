@@ -110,12 +110,12 @@ __global__ void __launch_bounds__(128, 4) kt_batch_lines_kernel(const __grid_con
     }
 }
 
-/* Mixed precision along y and eta: the face-once flux over line pieces of
+/* Mixed precision: the face-once flux over line pieces of
  * every member, one block per entry (member, block index among its face
  * blocks) -- flux_faces_lines, as the single-event
  * kt_flux_face_lines_kernel runs it. */
 template <int NQ, int EOS, int DIR>
-__global__ void __launch_bounds__(128, 5) kt_batch_face_lines_kernel(const __grid_constant__ BatchLaunch B)
+__global__ void __launch_bounds__(128, 4) kt_batch_face_lines_kernel(const __grid_constant__ BatchLaunch B)
 {
     __shared__ __align__(16) StageArgs sA;
     __shared__ double sm[NQ * 128];

@@ -49,7 +49,8 @@ BatchKernel batch_face_kernel_mixed(int nq, int eos_kind, int dir)
 template <int NQ, int EOS>
 static BatchKernel batch_face_lines_t(int dir)
 {
-    return dir == 3 ? kt_batch_face_lines_kernel<NQ, EOS, 3> : kt_batch_face_lines_kernel<NQ, EOS, 2>;
+    return dir == 1 ? kt_batch_face_lines_kernel<NQ, EOS, 1> : dir == 2 ? kt_batch_face_lines_kernel<NQ, EOS, 2>
+                                                                    : kt_batch_face_lines_kernel<NQ, EOS, 3>;
 }
 
 BatchKernel batch_face_lines_kernel_mixed(int nq, int eos_kind, int dir)

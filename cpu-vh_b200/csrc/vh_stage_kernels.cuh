@@ -280,12 +280,12 @@ static void launch_flux_face_lines(const StageArgs &a, cudaStream_t s)
 }
 
 /* mixed-precision flux form of the phase-split stage: VH_FACE_FORM=lines
- * (default: faces over line pieces along y and eta, 32 x 8 face tiles along
- * x, where a warp passes each face to the next lane by shuffle) or tiles
- * (32 x 8 face tiles along every axis).  131x131x61 Glauber event, ms per
- * step x/y/eta: lines 0.646/0.658/0.715, tiles 0.646/0.723/0.747; along x
- * line pieces measured 0.712 (a block barrier for the next face where the
- * tile's warp uses a shuffle), at 3 blocks per SM y/eta 0.744/0.803 */
+ * (default: faces over line pieces) or tiles (32 x 8 face tiles).  131x131x61
+ * Glauber event, us per launch x/y/eta: lines 216/213/222, tiles 252 along x
+ * (where a warp passes each face to the next lane by shuffle).  Lines staged in
+ * shared memory as the FP64 flux's measured 203/221/245: one face per thread
+ * leaves too little work between the block's barriers.  5 blocks per SM of 96
+ * registers: 231/235 along x/y. */
 static inline int face_form()
 {
     static int f = [] {
@@ -382,8 +382,7 @@ static void launch_stage_t(const StageArgs &a, cudaStream_t s, StageMarks *m)
     mark(0);
     if constexpr (MIXED) {
         if (face_form() != 0) {
-            const dim3 fb(kFaceTX, kFaceTY, 1);
-            launch_pdl(kt_flux_face_kernel<NQ, EOS, 1>, face_grid<1>(a), fb, 0, s, a);
+            launch_flux_face_lines<NQ, EOS, 1, 4>(a, s);
             mark(1);
             launch_flux_face_lines<NQ, EOS, 2, 4>(a, s);
             mark(2);
