@@ -423,15 +423,15 @@ __device__ __forceinline__ bool flow_pair(const DevEos &E, double t, const doubl
 }
 
 /* infer for one state in the same form; false: run infer */
-template <int EOS>
+template <int EOS, bool MIXED = false>
 __device__ __forceinline__ bool infer_direct(const DevEos &E, double t, double M0, double M1, double M2, double M3,
                                              double Pi, double ePrev, Prim &r)
 {
     const double M0s[1] = {M0}, M[1] = {M1 * M1 + M2 * M2 + t * t * M3 * M3}, Pis[1] = {Pi};
     double ef[1], yu, E2;
-    bool ok = energy_direct<EOS, 1, false>(E, M0s, M, Pis, ePrev, ef);
+    bool ok = energy_direct<EOS, 1, MIXED>(E, M0s, M, Pis, ePrev, ef);
     r.e = ef[0];
-    ok = flow_direct<EOS, false>(E, M0, Pi, r.e, r.p, r.ut, yu, E2) && ok;
+    ok = flow_direct<EOS, MIXED>(E, M0, Pi, r.e, r.p, r.ut, yu, E2) && ok;
     r.ux = M1 * E2;
     r.uy = M2 * E2;
     r.un = M3 * E2;
@@ -494,6 +494,7 @@ struct PlainQuot {
     __device__ __forceinline__ R rcp(R b) const { return R(1.0) / b; }
     __device__ __forceinline__ double deriv(double th, double x, double y, double z) const { return approx_deriv(th, x, y, z); }
 };
+template <bool MIXED = false>
 struct DirectQuot {
     unsigned key = ~0u;
     bool ok = true;
@@ -513,7 +514,7 @@ struct DirectQuot {
     __device__ __forceinline__ float root(float x)
     {
         ok = ok && in_range(x);
-        return sqrt_rn(x);
+        return root32<MIXED>(x);
     }
     __device__ __forceinline__ double deriv(double th, double x, double y, double z) const { return limited(th, x, y, z, 0x3ff00000); }
     __device__ __forceinline__ bool fine() const { return ok && key >= kDivKeyLo; }
@@ -527,14 +528,14 @@ struct DirectQuot {
 template <int EOS>
 __device__ __forceinline__ double temperature(PlainQuot &, const DevEos &E, double e) { return eos_T<EOS>(E, e); }
 template <int EOS>
-__device__ __forceinline__ double temperature(DirectQuot &dv, const DevEos &E, double e)
+__device__ __forceinline__ double temperature(DirectQuot<> &dv, const DevEos &E, double e)
 {
     dv.ok = dv.ok && in_range(e);
     if (EOS == 1) return floor15(eos_interp_direct(E, e, E.T_tb));
     return (double)powf_quarter(__double2float_rn(dv.over(e, E.a)), E.pq);
 }
 __device__ __forceinline__ double bulk_rate(PlainQuot &, const Zeta &Z, double a2, double T) { return 15 * a2 * T / zeta_over_s(Z, T); }
-__device__ __forceinline__ double bulk_rate(DirectQuot &dv, const Zeta &Z, double a2, double T)
+__device__ __forceinline__ double bulk_rate(DirectQuot<> &dv, const Zeta &Z, double a2, double T)
 {
     const double z = (T * 0.197326938 - Z.T0) / Z.w;
     const bool positive = Z.law != 1 || (Z.norm >= 0x1p-100 && z * z < 600.0);

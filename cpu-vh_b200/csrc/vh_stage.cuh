@@ -724,7 +724,7 @@ __device__ __forceinline__ void source_terms(Quot &dv, const StageArgs &A, long 
 template <int NQ, int EOS>
 __device__ __forceinline__ bool source_direct(const StageArgs &A, long long s, double *__restrict__ acc)
 {
-    DirectQuot dv;
+    DirectQuot<> dv;
     dv.ok = A.eos.direct && in_range(A.t) && in_range(A.dx) && in_range(A.dy) && in_range(A.dz) && in_range(A.etabar) &&
             in_range(2 * A.t);
     source_terms<NQ, EOS>(dv, A, s, acc);
@@ -783,7 +783,7 @@ __device__ __forceinline__ void regulation_factors(Quot &dv, double t, const dou
 
 /* When e > e_reg both factors are exactly 1 and the reference's multiplies are
  * identities, so the block is skipped. */
-template <int NQ, bool DIRECT = false>
+template <int NQ, bool DIRECT = false, bool MIXED = false>
 __device__ __forceinline__ void regulate(const StageArgs &A, double *__restrict__ acc, const Prim &P, bool &bad,
                                          long long s)
 {
@@ -794,7 +794,7 @@ __device__ __forceinline__ void regulate(const StageArgs &A, double *__restrict_
     }
     double facShear, facBulk;
     if constexpr (DIRECT) {
-        DirectQuot dv;
+        DirectQuot<MIXED> dv;
         regulation_factors<NQ>(dv, A.t_inf, acc, P, facShear, facBulk);
         if (!dv.fine() || !in_range(facShear) || !in_range(facBulk)) {
             PlainQuot pq;
@@ -817,7 +817,7 @@ __device__ __forceinline__ void regulate(const StageArgs &A, double *__restrict_
 
 /* (e, p, u) of the updated cell and its regulation, in the branch-free form
  * where it applies */
-template <int NQ, int EOS>
+template <int NQ, int EOS, bool MIXED>
 __device__ __forceinline__ Prim recover(const StageArgs &A, double *__restrict__ acc, double ePrev, bool &bad, long long s)
 {
     const double M0 = acc[0] - acc[4], M1 = acc[1] - acc[5], M2 = acc[2] - acc[6], M3 = acc[3] - acc[7];
@@ -826,9 +826,9 @@ __device__ __forceinline__ Prim recover(const StageArgs &A, double *__restrict__
     bool ranged = A.eos.direct != 0;
 #pragma unroll
     for (int n = 0; n < 8; ++n) ranged = ranged && state_ranged(acc[n]);
-    if (!(ranged && state_ranged(Pi)) || !infer_direct<EOS>(A.eos, A.t_inf, M0, M1, M2, M3, Pi, ePrev, P))
+    if (!(ranged && state_ranged(Pi)) || !infer_direct<EOS, MIXED>(A.eos, A.t_inf, M0, M1, M2, M3, Pi, ePrev, P))
         P = infer<EOS>(A.eos, A.t_inf, M0, M1, M2, M3, Pi, ePrev, bad);
-    regulate<NQ, true>(A, acc, P, bad, s);
+    regulate<NQ, true, MIXED>(A, acc, P, bad, s);
     return P;
 }
 
@@ -1495,14 +1495,7 @@ __device__ __forceinline__ void stage_faces_cell(const StageArgs &A, int i, int 
                 for (int n = 0; n < NQ; ++n) { acc[n] += __ldg(A.qbase + n * A.L + s); acc[n] /= 2; }
             }
         }
-        Prim P;
-        if constexpr (MIXED) {
-            P = infer<EOS, true>(A.eos, A.t_inf, acc[0] - acc[4], acc[1] - acc[5], acc[2] - acc[6], acc[3] - acc[7],
-                                 (NQ == 15) ? acc[14] : 0.0, ePrev, bad);
-            regulate<NQ>(A, acc, P, bad, s);
-        } else {
-            P = recover<NQ, EOS>(A, acc, ePrev, bad, s);
-        }
+        const Prim P = recover<NQ, EOS, MIXED>(A, acc, ePrev, bad, s);
         put_with_ghosts<NQ>(A, i, j, k, s, acc, P);
     }
     if (bad) raise_error(A.err, kErrNan, s, A.step);
