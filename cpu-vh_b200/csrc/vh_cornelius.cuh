@@ -287,6 +287,33 @@ static __device__ void poly_normal(const WorkRef &w, Poly &p, double *normal)
         for (int j = 0; j < D; j++) normal[j] += acc[i][j];
 }
 
+/* Cube::construct_polygons (cornelius.cpp:1580-1622): a cube's lines first ..
+ * first + nlines - 1 into polygons -- one of all lines, or chains of touching
+ * lines where the cube is ambiguous */
+static __device__ void chain_polygons(WorkRef &w, int first, int nlines, int const_i, bool ambiguous)
+{
+    if (ambiguous) {
+        bool not_used[12];
+        int used = 0;
+        for (int i = 0; i < nlines; i++) not_used[i] = true;
+        do {
+            if (nlines - used < 3 || w.np >= w.pcap) { w.error = true; return; }
+            Poly &p = w.poly[w.np];
+            poly_init(p, const_i);
+            for (int i = 0; i < nlines; i++)
+                if (not_used[i] && poly_add_line(w, p, first + i, false)) { not_used[i] = false; used++; i = 0; }
+            if (w.error) return;
+            w.np++;
+        } while (used < nlines);
+    } else {
+        if (w.np >= w.pcap) { w.error = true; return; }
+        Poly &p = w.poly[w.np];
+        poly_init(p, const_i);
+        for (int i = 0; i < nlines; i++) poly_add_line(w, p, first + i, true);
+        w.np++;
+    }
+}
+
 /* Cube::split_to_squares + construct_polygons + check_ambiguous
  * (cornelius.cpp:1502-1650).  Returns the cube's number of lines; its
  * polygons are appended to w.poly, and *ambiguous reports the cube flag. */
@@ -316,26 +343,7 @@ static __device__ int cube_polygons(WorkRef &w, const double cube[2][2][2], int 
     if (nlines == 0) return 0;
     if (amb == 0 && nlines == 6) amb++;
     *ambiguous = amb > 0;
-    if (amb > 0) {
-        bool not_used[12];
-        int used = 0;
-        for (int i = 0; i < nlines; i++) not_used[i] = true;
-        do {
-            if (nlines - used < 3 || w.np >= w.pcap) { w.error = true; return nlines; }
-            Poly &p = w.poly[w.np];
-            poly_init(p, const_i);
-            for (int i = 0; i < nlines; i++)
-                if (not_used[i] && poly_add_line(w, p, first + i, false)) { not_used[i] = false; used++; i = 0; }
-            if (w.error) return nlines;
-            w.np++;
-        } while (used < nlines);
-    } else {
-        if (w.np >= w.pcap) { w.error = true; return nlines; }
-        Poly &p = w.poly[w.np];
-        poly_init(p, const_i);
-        for (int i = 0; i < nlines; i++) poly_add_line(w, p, first + i, true);
-        w.np++;
-    }
+    chain_polygons(w, first, nlines, const_i, amb > 0);
     return nlines;
 }
 

@@ -325,27 +325,147 @@ __device__ __forceinline__ void put_count(const FoScratch &sc, int c, int ne)
     atomicAdd(sc.csum + c / kScanChunk, ne);
 }
 
-/* 2+1D: one thread per cube, one warp per block (the few hundred crossed cubes
- * of an event spread over the SMs) */
-__global__ void __launch_bounds__(32) fo_count_kernel(const __grid_constant__ FoArgs a, FoScratch sc)
+/* 2+1D: eight lanes per cube, sixteen cubes per block.  One thread per cube is
+ * one thread's latency through its squares, polygons and sums (20-26 us whatever
+ * the number of cubes).  Here lane q < 6 cuts the q-th square (cube_polygons'
+ * order; its lines go after the lanes before it), one lane chains the polygons
+ * where that is ambiguous, and the sums of Polygon::calculate_centroid and
+ * calculate_normal (cornelius.cpp:478-617) run a line per lane, added in the
+ * reference's order through width-8 shuffles: the same elements. */
+constexpr int kG3 = 16;                       /* cubes per 128-thread block */
+constexpr int kC3Lines = 12, kC3Polys = 4;     /* 6 squares x 2 lines; a polygon has at least 3 */
+struct Count3Shared {
+    double p[kG3][kC3Lines][2][4];
+    double out[kG3][kC3Lines][4];
+    unsigned char flip[kG3][kC3Lines];
+    cor::Poly poly[kG3][kC3Polys];
+    int np[kG3];
+};
+
+/* adds the lanes' terms v[0..n) of items r .. r + 7 (those below count) to sum, in item order */
+template <int N>
+__device__ __forceinline__ void add_in_order(unsigned gmask, const double (&v)[N], double (&sum)[N], int r, int count)
 {
+    for (int u = 0; u < 8; u++) {
+        double t[N];
+#pragma unroll
+        for (int k = 0; k < N; k++) t[k] = __shfl_sync(gmask, v[k], u, 8);
+        if (r + u < count)
+#pragma unroll
+            for (int k = 0; k < N; k++) sum[k] += t[k];
+    }
+}
+
+__global__ void __launch_bounds__(128) fo_count3_kernel(const __grid_constant__ FoArgs a, FoScratch sc)
+{
+    __shared__ Count3Shared S;
     dep_wait();
     dep_trigger();
     const int nst = sc.hdr[0];
-    for (int i = blockIdx.x * 32 + threadIdx.x; i < nst; i += gridDim.x * 32) {
+    const int tid = threadIdx.x, g = tid >> 3, q = tid & 7, lane = tid & 31;
+    const unsigned gmask = 0xFFu << (lane & ~7);
+    const double dx[4] = {1, a.dtau_c, a.dx, a.dy};
+    for (int i = blockIdx.x * kG3 + g; i < nst; i += gridDim.x * kG3) {
         const int c = sc.list[i];
         int ix, iy, iz;
         cube_coords(a, c, ix, iy, iz);
-        cor::Work w;
-        double cen[cor::kMaxHedra][4], nor[cor::kMaxHedra][4];
-        int ne = cube_surface(a, ix, iy, iz, w, cen, nor);
-        if (ne < 0) { raise_error(a.err, 5, c, a.n); ne = 0; }
-        put_count(sc, c, ne);
-        if (i < a.slot_cap) {
-            double *o = a.slots + (long long)i * kSlotDoubles;
-            for (int k = 0; k < ne; k++)
-                for (int d = 0; d < 4; d++) { o[8 * k + d] = cen[k][d]; o[8 * k + 4 + d] = nor[k][d]; }
+        double cu[2][2][2];
+        for (int t = 0; t < 2; t++) for (int bx = 0; bx < 2; bx++) for (int by = 0; by < 2; by++)
+            cu[t][bx][by] = slab(a, t, 0, ix + bx, iy + by, 0);
+        /* this lane's square: axis 1 + q/2 held at its lower or upper end */
+        const int axis = 1 + (q >> 1), end = q & 1;
+        double sq[2][2];
+        int nl = 0;
+        bool err = false;
+        if (q < 6) {
+            for (int A = 0; A < 2; A++)
+                for (int B = 0; B < 2; B++)
+                    sq[A][B] = (axis == 1) ? (end ? cu[1][A][B] : cu[0][A][B])
+                             : (axis == 2) ? (end ? cu[A][1][B] : cu[A][0][B]) : (end ? cu[A][B][1] : cu[A][B][0]);
+            const int nc = cor::square_cut_count(sq, a.eF);
+            err = nc != 0 && nc != 2 && nc != 4;
+            nl = err ? 0 : nc / 2;
         }
+        int incl = nl;
+        for (int o = 1; o < 8; o <<= 1) {
+            const int v = __shfl_up_sync(gmask, incl, o, 8);
+            if (q >= o) incl += v;
+        }
+        const int nlines = __shfl_sync(gmask, incl, 7, 8), at = incl - nl;
+        if (nl > 0) {
+            cor::WorkRef w{S.p[g], S.out[g], S.flip[g], S.poly[g], at, 0, at + nl, kC3Polys, false};
+            cor::square_lines(w, sq, 0, axis, 0, end * dx[axis], a.eF, dx);
+            err = err || w.error || w.nl != at + nl;
+        }
+        bool ambiguous = (__ballot_sync(gmask, nl == 2) & gmask) != 0 || nlines == 6;
+        err = (__ballot_sync(gmask, err) & gmask) != 0;
+        __syncwarp(gmask);
+        if (q == 0) {
+            cor::WorkRef w{S.p[g], S.out[g], S.flip[g], S.poly[g], nlines, 0, kC3Lines, kC3Polys, false};
+            if (!err && nlines > 0) cor::chain_polygons(w, 0, nlines, 0, ambiguous);
+            S.np[g] = (err || w.error) ? -1 : w.np;
+        }
+        __syncwarp(gmask);
+        const int np = S.np[g];
+        const cor::WorkRef w{S.p[g], S.out[g], S.flip[g], S.poly[g], nlines, np, kC3Lines, kC3Polys, false};
+        for (int k = 0; k < np; k++) {
+            const cor::Poly &P = S.poly[g][k];
+            const int n = P.nlines;
+            double mean[4] = {0, 0, 0, 0}, cen[4], nor[4] = {0, 0, 0, 0};
+            for (int r = 0; r < n; r += 8) {
+                double v[4] = {0, 0, 0, 0};
+                if (r + q < n) {
+                    const double *p1 = cor::lstart(w, P.line[r + q]), *p2 = cor::lend(w, P.line[r + q]);
+                    for (int j = 0; j < 4; j++) v[j] = p1[j] + p2[j];
+                }
+                add_in_order<4>(gmask, v, mean, r, n);
+            }
+            for (int j = 0; j < 4; j++) cen[j] = mean[j] = mean[j] / (double)(2.0 * n);
+            if (n != 3) {
+                double up[5] = {0, 0, 0, 0, 0};                 /* centroid sums, then the area */
+                for (int r = 0; r < n; r += 8) {
+                    double v[5] = {0, 0, 0, 0, 0};
+                    if (r + q < n) {
+                        const double *p1 = cor::lstart(w, P.line[r + q]), *p2 = cor::lend(w, P.line[r + q]);
+                        double cm[4], d1[4], d2[4];
+                        for (int j = 0; j < 4; j++) cm[j] = (p1[j] + p2[j] + mean[j]) / 3.0;
+                        for (int j = 0; j < 4; j++) { d1[j] = p1[j] - mean[j]; d2[j] = p2[j] - mean[j]; }
+                        const double s1 = d1[2] * d2[3] - d1[3] * d2[2];
+                        const double s2 = d1[1] * d2[3] - d1[3] * d2[1];
+                        const double s3 = d1[2] * d2[1] - d1[1] * d2[2];
+                        const double A = 0.5 * sqrt(s1 * s1 + s2 * s2 + s3 * s3);
+                        for (int j = 0; j < 4; j++) v[j] = cm[j] * A;
+                        v[4] = A;
+                    }
+                    add_in_order<5>(gmask, v, up, r, n);
+                }
+                for (int j = 0; j < 4; j++) cen[j] = up[j] / up[4];
+            }
+            for (int r = 0; r < n; r += 8) {
+                double v[4] = {0, 0, 0, 0};
+                if (r + q < n) {
+                    const int l = P.line[r + q];
+                    const double *p1 = cor::lstart(w, l), *p2 = cor::lend(w, l);
+                    double d1[4], d2[4], vout[4];
+                    for (int j = 0; j < 4; j++) { d1[j] = p1[j] - cen[j]; d2[j] = p2[j] - cen[j]; }
+                    v[1] = 0.5 * (d1[2] * d2[3] - d1[3] * d2[2]);
+                    v[2] = -0.5 * (d1[1] * d2[3] - d1[3] * d2[1]);
+                    v[3] = 0.5 * (d1[1] * d2[2] - d1[2] * d2[1]);
+                    for (int j = 0; j < 4; j++) vout[j] = w.out[l][j] - cen[j];
+                    cor::orient(v, vout);
+                }
+                add_in_order<4>(gmask, v, nor, r, n);
+            }
+            if (q == 0 && i < a.slot_cap) {
+                double *o = a.slots + (long long)i * kSlotDoubles + 8 * k;
+                for (int d = 0; d < 4; d++) { o[d] = cen[d]; o[4 + d] = nor[d]; }
+            }
+        }
+        if (q == 0) {
+            if (np < 0) raise_error(a.err, 5, c, a.n);
+            else put_count(sc, c, np);
+        }
+        __syncwarp(gmask);
     }
 }
 
@@ -828,7 +948,7 @@ void launch_freezeout(const FoArgs &a, cudaStream_t st)
     const unsigned N = (unsigned)a.nx * a.ny * a.nz;
     launch_dep(fo_open_kernel, (N + 255) / 256, 256, 0, st, a, sc);
     if (a.nz > 1) launch_count4(a, sc, st);
-    else launch_dep(fo_count_kernel, (unsigned)std::min((sc.nc + 31) / 32, 148 * 16), 32, 0, st, a, sc);
+    else launch_dep(fo_count3_kernel, (unsigned)std::min((sc.nc + kG3 - 1) / kG3, 148 * 8), 128, 0, st, a, sc);
     launch_dep(fo_offsets_kernel, (unsigned)sc.nb, kScanThreads, 0, st, sc, a.host_hdr);
     launch_freezeout_emit(a, st);
 }
