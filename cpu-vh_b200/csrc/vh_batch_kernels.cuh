@@ -42,8 +42,8 @@ __global__ void __launch_bounds__(128, PHASE == 0 && !MIXED ? 3 : 4) kt_batch_ke
         } else if constexpr (PHASE >= 1 && PHASE <= 3) {
             flux_phase<NQ, EOS, PHASE, MIXED>(sA, s);
         } else if constexpr (PHASE == 4) {
-            if (ZM == 1 || (ZM == 2 && sA.nz > 1)) final_body<NQ, EOS, true, STAGE2>(sA, i, j, k, s);
-            else final_body<NQ, EOS, false, STAGE2>(sA, i, j, k, s);
+            if (ZM == 1 || (ZM == 2 && sA.nz > 1)) final_body<NQ, EOS, true, STAGE2, MIXED>(sA, i, j, k, s);
+            else final_body<NQ, EOS, false, STAGE2, MIXED>(sA, i, j, k, s);
         } else {
             if (ZM == 1 || (ZM == 2 && sA.nz > 1)) stage_phase<NQ, EOS, true, STAGE2, MIXED>(sA, i, j, k, s);
             else stage_phase<NQ, EOS, false, STAGE2, MIXED>(sA, i, j, k, s);

@@ -759,25 +759,27 @@ __device__ __forceinline__ void regulation_factors(Quot &dv, double t, const dou
     double piu1 = -(pixn * t2 * un) + pitx * ut - pixx * ux - pixy * uy;
     double piu2 = -(piyn * t2 * un) + pity * ut - pixy * ux - piyy * uy;
     double piu3 = -(pinn * t2 * un) + pitn * ut - pixn * ux - piyn * uy;
-    /* the divisions by rhomax = 1 of the source are exact and left out */
+    /* the divisions by rhomax = 1 of the source are exact and left out.  The
+     * five quotients X / xi0 / spipi share a positive divisor, and rounding is
+     * monotone, so their maximum is the quotient of the largest X (a NaN is
+     * passed over by fmax on either side of the division) */
     static_assert(rhomax == 1.0, "");
-    const double ys = dv.rcp(spipi);
-    double a1 = dv.over(spipi, (double)dv.root(__double2float_rn(P.e * P.e + 3 * P.p * P.p)));
-    double a2 = dv.quotient(dv.over_const(pimumu, xi0, 1.0 / xi0), spipi, ys);
-    double a3 = dv.quotient(dv.over_const(piu0, xi0, 1.0 / xi0), spipi, ys);
-    double a4 = dv.quotient(dv.over_const(piu1, xi0, 1.0 / xi0), spipi, ys);
-    double a5 = dv.quotient(dv.over_const(piu2, xi0, 1.0 / xi0), spipi, ys);
-    double a6 = dv.quotient(dv.over_const(piu3, xi0, 1.0 / xi0), spipi, ys);
-    double a12 = fmax(a1, a2), a34 = fmax(a3, a4), a56 = fmax(a5, a6), a3456 = fmax(a34, a56);
-    double rho = fmax(a12, a3456);
+    const double a1 = dv.over(spipi, (double)dv.root(__double2float_rn(P.e * P.e + 3 * P.p * P.p)));
+    double rho;
+    if (spipi > 0 && spipi < 1e300) {
+        const double X = fmax(fmax(pimumu, fmax(piu0, piu1)), fmax(piu2, piu3));
+        rho = fmax(a1, dv.over(dv.over_const(X, xi0, 1.0 / xi0), spipi));
+    } else {
+        const double a2 = pimumu / xi0 / spipi, a3 = piu0 / xi0 / spipi, a4 = piu1 / xi0 / spipi;
+        const double a5 = piu2 / xi0 / spipi, a6 = piu3 / xi0 / spipi;
+        rho = fmax(fmax(a1, a2), fmax(fmax(a3, a4), fmax(a5, a6)));
+    }
     auto over = [&](double a, double b) { return dv.over(a, b); };
-    facShear = dv.over(vh_tanh(rho, over), rho);
-    if (fabs(rho) < 1.e-7) facShear = 1.0;
-    facBulk = 1.0;
+    facShear = facBulk = 1.0;                  /* below 1e-7 the reference sets 1 */
+    if (!(fabs(rho) < 1.e-7)) facShear = dv.over(vh_tanh(rho, over), rho);
     if (NQ == 15) {
         double rhoBulk = dv.over(fabs(Pi), P.p);
-        facBulk = dv.over(vh_tanh(rhoBulk, over), rhoBulk);
-        if (fabs(rhoBulk) < 1.e-7) facBulk = 1.0;
+        if (!(fabs(rhoBulk) < 1.e-7)) facBulk = dv.over(vh_tanh(rhoBulk, over), rhoBulk);
     }
 }
 
@@ -942,7 +944,7 @@ __device__ __forceinline__ void flux_body(const StageArgs &A, long long s)
     if (bad) raise_error(A.err, kErrNan, s, A.step);
 }
 
-template <int NQ, int EOS, bool HAS_Z, bool STAGE2>
+template <int NQ, int EOS, bool HAS_Z, bool STAGE2, bool MIXED>
 __device__ __forceinline__ void final_body(const StageArgs &A, int i, int j, int k, long long s)
 {
     const double ePrev = __ldg(A.ein + s);
@@ -958,9 +960,14 @@ __device__ __forceinline__ void final_body(const StageArgs &A, int i, int j, int
 #pragma unroll
         for (int n = 0; n < NQ; ++n) { acc[n] += __ldg(A.qbase + n * A.L + s); acc[n] /= 2; }
     }
-    Prim P = infer<EOS, true>(A.eos, A.t_inf, acc[0] - acc[4], acc[1] - acc[5], acc[2] - acc[6], acc[3] - acc[7],
-                              (NQ == 15) ? acc[14] : 0.0, ePrev, bad);
-    regulate<NQ>(A, acc, P, bad, s);
+    Prim P;
+    if constexpr (MIXED) {
+        P = infer<EOS, true>(A.eos, A.t_inf, acc[0] - acc[4], acc[1] - acc[5], acc[2] - acc[6], acc[3] - acc[7],
+                             (NQ == 15) ? acc[14] : 0.0, ePrev, bad);
+        regulate<NQ>(A, acc, P, bad, s);
+    } else {
+        P = recover<NQ, EOS, false>(A, acc, ePrev, bad, s);
+    }
     if (bad) raise_error(A.err, kErrNan, s, A.step);
     put_with_ghosts<NQ>(A, i, j, k, s, acc, P);
 }

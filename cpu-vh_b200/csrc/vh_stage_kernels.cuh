@@ -303,10 +303,17 @@ static inline dim3 face_grid(const StageArgs &a)
     return dim3((a.nx + kFaceTX - 1) / kFaceTX, a.ny, (a.nz + kFaceTY - 2) / (kFaceTY - 1));
 }
 
-/* MIXED is part of the kernel's name although the body is the same: the
- * FP64 and the mixed translation units compile it with different
- * floating-point flags, and one name for two different device functions
- * would leave it to the runtime which of the two a launch runs */
+/* Memory-bound (31 values read and 21 written per cell in stage 2; 76 us per
+ * 131x131x61 launch with nothing computed).  Most cells lie in the dilute
+ * edge, whose regulation held the warps: five quotients by one divisor and
+ * their maximum are now the maximum's quotient, and the tanh is left out where
+ * the reference overrides it with 1: 109 -> 93 us (stage 1: 99 -> 86).  (Walking
+ * the lattice with resident blocks that request the next cell first measured
+ * 132 us: 12 warps per SM.)
+ * MIXED is part of the kernel's name: the FP64 and the mixed translation units
+ * compile it with different floating-point flags, and one name for two
+ * different device functions would leave it to the runtime which of the two a
+ * launch runs */
 template <int NQ, int EOS, bool HAS_Z, bool STAGE2, bool MIXED>
 __global__ void __launch_bounds__(128, VH_STAGE_MIN_BLOCKS) kt_final_kernel(const __grid_constant__ StageArgs A)
 {
@@ -315,7 +322,7 @@ __global__ void __launch_bounds__(128, VH_STAGE_MIN_BLOCKS) kt_final_kernel(cons
     int i, j, k;
     long long s;
     if (!stage_cell_flat(A, i, j, k, s)) return;
-    final_body<NQ, EOS, HAS_Z, STAGE2>(A, i, j, k, s);
+    final_body<NQ, EOS, HAS_Z, STAGE2, MIXED>(A, i, j, k, s);
 }
 
 /* Fused (face-parallel) for small lattices, which are latency-bound;
