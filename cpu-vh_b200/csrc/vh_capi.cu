@@ -187,6 +187,7 @@ int vh_event_destroy(vh_event *ev)
         cudaStreamSynchronize(ev->stream);
     }
     if (ev->fo_hdr) cudaFreeHost(ev->fo_hdr);
+    if (ev->fo_host) cudaFreeHost(ev->fo_host);
     if (ev->fo_done) cudaEventDestroy(ev->fo_done);
     for (auto &m : ev->marks)
         for (cudaEvent_t e : m.ev) cudaEventDestroy(e);
@@ -607,6 +608,8 @@ static void fo_args(vh_event *ev, vh::FoArgs &a)
     a.err.code = ev->err; a.err.step = ev->err + 1; a.err.cell = ev->err_cell;
     a.counts = ev->fo_scratch;
     a.host_hdr = ev->fo_hdr;
+    a.host_elems = ev->fo_host;
+    a.host_cap = vh::kFoHostElems;
     a.elems = ev->fo_elems;
     a.cap = ev->fo_cap;
     a.slots = ev->fo_slots;
@@ -628,6 +631,7 @@ int vh_event_freezeout_launch(vh_event *ev)
         CUDA_TRY(cudaMemsetAsync(ev->fo_scratch + ev->fo_scratch_ints - vh::kFoHeaderInts, 0, vh::kFoHeaderInts * sizeof(int),
                                  ev->stream));
         CUDA_TRY(cudaMallocHost(&ev->fo_hdr, 2 * sizeof(int)));
+        CUDA_TRY(cudaMallocHost(&ev->fo_host, (size_t)vh::kFoHostElems * VH_FO_COLUMNS * sizeof(double)));
         CUDA_TRY(cudaEventCreateWithFlags(&ev->fo_done, cudaEventDisableTiming));
         /* a first element buffer sized for a surface crossing the lattice
          * (twice its cross sections in 3+1D, eight times its edges in 2+1D),
@@ -695,6 +699,10 @@ int vh_event_fetch_surface(vh_event *ev, double *host_out, int cap_elements, int
     if (ev->fo_count > cap_elements) return fail(VH_ERR_CAPACITY, "surface buffer too small");
     if (ev->fo_count == 0) return VH_OK;
     if (!host_out) return fail(VH_ERR_ARG, "null output");
+    if (ev->fo_count <= vh::kFoHostElems && !ev->fo_pending) {
+        std::memcpy(host_out, ev->fo_host, (size_t)ev->fo_count * VH_FO_COLUMNS * sizeof(double));
+        return VH_OK;
+    }
     CUDA_TRY(cudaMemcpyAsync(host_out, ev->fo_elems, (size_t)ev->fo_count * VH_FO_COLUMNS * sizeof(double),
                              cudaMemcpyDeviceToHost, ev->stream));
     CUDA_TRY(cudaStreamSynchronize(ev->stream));

@@ -71,6 +71,7 @@ struct vh_event {
     double *fo_slots = nullptr;           /* element slots of the count step (vh_fo.cu) */
     int fo_slot_cap = 0;
     int fo_count = 0;
+    double *fo_host = nullptr;            /* pinned: the last block's first kFoHostElems elements */
     int *fo_hdr = nullptr;                /* pinned: n_above, n_total of the last block */
     cudaEvent_t fo_done = nullptr;
     bool fo_pending = false;              /* launched, not yet finished */

@@ -860,7 +860,10 @@ static __device__ __noinline__ void emit_recompute(const FoArgs &a, int ix, int 
     const int ne = cube_surface(a, ix, iy, iz, w, cen, nor);
     for (int k = 0; k < ne; k++) {
         if (off + k >= a.cap) return;
-        emit_element<EOS>(a, ix, iy, iz, cen[k], nor[k], a.elems + (off + k) * VH_FO_COLUMNS);
+        double *o = a.elems + (off + k) * VH_FO_COLUMNS;
+        emit_element<EOS>(a, ix, iy, iz, cen[k], nor[k], o);
+        if (off + k < a.host_cap)
+            for (int j = 0; j < VH_FO_COLUMNS; j++) a.host_elems[(off + k) * VH_FO_COLUMNS + j] = o[j];
     }
 }
 
@@ -868,9 +871,13 @@ static __device__ __noinline__ void emit_recompute(const FoArgs &a, int ix, int 
  * holds e, also T and P), one coordinate of position and normal each (10-13) */
 template <int EOS>
 __device__ __forceinline__ void emit_lane(const FoArgs &a, int ix, int iy, int iz, const double *cen, const double *nor,
-                                          double *__restrict__ o, int lane)
+                                          double *__restrict__ o, double *__restrict__ host, int lane)
 {
     const bool four = a.nz > 1;
+    auto put = [&](int col, double x) {
+        o[col] = x;
+        if (host) host[col] = x;
+    };
     if (lane < 10) {
         const int v = lane;
         double f;
@@ -894,10 +901,10 @@ __device__ __forceinline__ void emit_lane(const FoArgs &a, int ix, int iy, int i
                         slab(a, 1, v + 1, ix + 1, iy, 0), slab(a, 1, v + 1, ix, iy + 1, 0),
                         slab(a, 0, v + 1, ix + 1, iy + 1, 0), slab(a, 1, v + 1, ix + 1, iy + 1, 0));
         }
-        o[v < 4 ? 8 + v : 10 + v] = f;
+        put(v < 4 ? 8 + v : 10 + v, f);
         if (v == 3) {
-            o[12] = eos_T<EOS>(a.eos, f);
-            o[13] = eos_p<EOS>(a.eos, f);
+            put(12, eos_T<EOS>(a.eos, f));
+            put(13, eos_p<EOS>(a.eos, f));
         }
     } else if (lane < 14) {
         const int d = lane - 10, n = (d == 0) ? 0 : (d == 1) ? a.nx : (d == 2) ? a.ny : a.nz;
@@ -905,11 +912,11 @@ __device__ __forceinline__ void emit_lane(const FoArgs &a, int ix, int iy, int i
         const double h = (d == 1) ? a.dx : (d == 2) ? a.dy : a.dz;
         const double cell = (d == 0) ? a.t0 + ((double)a.n) * a.dt : (double)i * h - (((double)(n - 1)) / 2.0 * h);
         if (four) {
-            o[d] = cen[d] + cell;
-            o[4 + d] = a.t * nor[d];
+            put(d, cen[d] + cell);
+            put(4 + d, a.t * nor[d]);
         } else {
-            o[d] = (d < 3) ? cen[d + 1] + cell : 0.0;
-            o[4 + d] = (d < 3) ? a.t * nor[d + 1] : 0.0;
+            put(d, (d < 3) ? cen[d + 1] + cell : 0.0);
+            put(4 + d, (d < 3) ? a.t * nor[d + 1] : 0.0);
         }
     }
 }
@@ -931,7 +938,8 @@ __global__ void __launch_bounds__(128) fo_emit_kernel(const __grid_constant__ Fo
         const int ne = sc.counts[c + 1] - (int)off;
         const double *sl = a.slots + (long long)i * kSlotDoubles;
         for (int k = 0; k < ne && off + k < a.cap; k++)
-            emit_lane<EOS>(a, ix, iy, iz, sl + 8 * k, sl + 8 * k + 4, a.elems + (off + k) * VH_FO_COLUMNS, lane);
+            emit_lane<EOS>(a, ix, iy, iz, sl + 8 * k, sl + 8 * k + 4, a.elems + (off + k) * VH_FO_COLUMNS,
+                           off + k < a.host_cap ? a.host_elems + (off + k) * VH_FO_COLUMNS : nullptr, lane);
     }
     /* cubes beyond the slots: a thread each */
     for (int i = kept + blockIdx.x * 128 + threadIdx.x; i < nst; i += gridDim.x * 128) {

@@ -145,11 +145,18 @@ struct FoArgs {
     int cap;                     /* capacity of elems in elements */
     double *slots;               /* centroids and normals of the first slot_cap crossed cubes */
     int slot_cap;
+    double *host_elems;          /* pinned: the first host_cap elements, for a host that reads a small surface */
+    int host_cap;
 };
 
 /* doubles of one crossed cube's element slot: up to 10 elements (Cornelius
  * MAX_ELEMENTS), centroid and normal (4 + 4) each */
 constexpr int kFoSlotDoubles = 80;
+/* a block's first elements also go to pinned host memory: a small surface (a
+ * 2+1D event's, a late block's) is then read without a copy and a second wait
+ * for the stream, 10 us of a 33x29 event's block */
+constexpr int kFoHostElems = 512;
+
 /* the freezeout scratch ends with its header, zero before the first block */
 constexpr int kFoHeaderInts = 4;
 

@@ -28,6 +28,7 @@ namespace vh {
 
 /* DynamicalVariables.cpp:169-218 (T^{tau mu} from e, p+Pi, u, pi) and the
  * ghost faces; the previous-step velocity starts equal to u. */
+template <int NQ>
 __global__ void init_kernel(const __grid_constant__ InitArgs A)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -41,16 +42,18 @@ __global__ void init_kernel(const __grid_constant__ InitArgs A)
     double qv[15];
     const double e = A.e[m], p = A.p[m];
     const double ut = A.u[m], ux = A.u[N + m], uy = A.u[2 * N + m], un = A.u[3 * N + m];
+#pragma unroll
     for (int c = 0; c < 10; ++c) qv[4 + c] = A.pi ? A.pi[c * N + m] : 0.0;
-    const double Pi = (A.nq == 15 && A.Pi) ? A.Pi[m] : 0.0;
-    if (A.nq == 15) qv[14] = Pi;
+    const double Pi = (NQ == 15 && A.Pi) ? A.Pi[m] : 0.0;
+    qv[14] = Pi;
     const double P = p + Pi;
     qv[0] = (e + P) * ut * ut - P + qv[4];
     qv[1] = (e + P) * ut * ux + qv[5];
     qv[2] = (e + P) * ut * uy + qv[6];
     qv[3] = (e + P) * ut * un + qv[7];
     auto put = [&](long long d) {
-        for (int n = 0; n < A.nq; ++n) A.q[n * L + d] = qv[n];
+#pragma unroll
+        for (int n = 0; n < NQ; ++n) A.q[n * L + d] = qv[n];
         A.eo[d] = e; A.po[d] = p;
         A.uo[d] = ut; A.uo[L + d] = ux; A.uo[2 * L + d] = uy; A.uo[3 * L + d] = un;
     };
@@ -215,7 +218,8 @@ void launch_init(const InitArgs &a, cudaStream_t s)
 {
     dim3 block(32, 4, 1);
     dim3 grid((a.nx + 31) / 32, (a.ny + 3) / 4, a.nz);
-    init_kernel<<<grid, block, 0, s>>>(a);
+    if (a.nq == 15) init_kernel<15><<<grid, block, 0, s>>>(a);
+    else init_kernel<14><<<grid, block, 0, s>>>(a);
 }
 
 int stage_launches(int nx, int ny, int nz, bool mixed)
