@@ -126,75 +126,86 @@ __device__ __forceinline__ int square_cut_count(const double P[2][2], double E0)
     return nc;
 }
 
-/* Square::construct_lines with ends_of_edge and find_outside
- * (cornelius.cpp:1134-1337); appends its lines to w. */
-static __device__ void square_lines(WorkRef &w, const double P[2][2], int c0, int c1, double v0_, double v1_, double E0, const double *dx)
+/* element i of a 4-vector held in registers (an index known only at run time
+ * would move the vector to local memory) */
+__device__ __forceinline__ double pick(const double *v, int i) { return (i < 2) ? (i == 0 ? v[0] : v[1]) : (i == 2 ? v[2] : v[3]); }
+
+/* where the threshold cuts the edge from corner value A to B (ends_of_edge,
+ * cornelius.cpp:1170-1235): at t of its length d */
+__device__ __forceinline__ bool edge_cut(double A, double B, double E0, double d, double &t)
 {
-    int above = 0;
-    for (int i = 0; i < 2; i++)
-        for (int j = 0; j < 2; j++)
-            if (P[i][j] >= E0) above++;
+    if ((A - E0) * (B - E0) < 0) { t = (A - E0) / (A - B) * d; return true; }
+    if (A == E0 && B < E0) { t = 1e-9 * d; return true; }
+    if (B == E0 && A < E0) { t = (1.0 - 1e-9) * d; return true; }
+    return false;
+}
+
+/* Square::construct_lines with ends_of_edge and find_outside
+ * (cornelius.cpp:1134-1337); appends its lines to w.  The cuts stay in
+ * registers: the four edges in the reference's order, of which two or four
+ * are cut. */
+static __device__ __forceinline__ void square_lines(WorkRef &w, const double P[2][2], int c0, int c1, double v0_, double v1_, double E0, const double *dx)
+{
+    const int above = (P[0][0] >= E0) + (P[0][1] >= E0) + (P[1][0] >= E0) + (P[1][1] >= E0);
     if (above == 0 || above == 4) return;
-    int x1 = -1, x2 = -1;
-    for (int i = 0; i < D; i++)
-        if (i != c0 && i != c1) { if (x1 < 0) x1 = i; else x2 = i; }
-    const double d1 = dx[x1], d2 = dx[x2];
-    double cuts[4][2], out[2][2];
-    int nc = 0;
-#define CUT(a, b) do { cuts[nc][0] = (a); cuts[nc][1] = (b); nc++; } while (0)
-    if ((P[0][0] - E0) * (P[1][0] - E0) < 0) CUT((P[0][0] - E0) / (P[0][0] - P[1][0]) * d1, 0);
-    else if (P[0][0] == E0 && P[1][0] < E0) CUT(1e-9 * d1, 0);
-    else if (P[1][0] == E0 && P[0][0] < E0) CUT((1.0 - 1e-9) * d1, 0);
-    if ((P[0][0] - E0) * (P[0][1] - E0) < 0) CUT(0, (P[0][0] - E0) / (P[0][0] - P[0][1]) * d2);
-    else if (P[0][0] == E0 && P[0][1] < E0) CUT(0, 1e-9 * d2);
-    else if (P[0][1] == E0 && P[0][0] < E0) CUT(0, (1.0 - 1e-9) * d2);
-    if ((P[1][0] - E0) * (P[1][1] - E0) < 0) CUT(d1, (P[1][0] - E0) / (P[1][0] - P[1][1]) * d2);
-    else if (P[1][0] == E0 && P[1][1] < E0) CUT(d1, 1e-9 * d2);
-    else if (P[1][1] == E0 && P[1][0] < E0) CUT(d1, (1.0 - 1e-9) * d2);
-    if ((P[0][1] - E0) * (P[1][1] - E0) < 0) CUT((P[0][1] - E0) / (P[0][1] - P[1][1]) * d1, d2);
-    else if (P[0][1] == E0 && P[1][1] < E0) CUT(1e-9 * d1, d2);
-    else if (P[1][1] == E0 && P[0][1] < E0) CUT((1.0 - 1e-9) * d1, d2);
-#undef CUT
+    const int x1 = (c0 != 0 && c1 != 0) ? 0 : (c0 != 1 && c1 != 1) ? 1 : 2;
+    const int x2 = (c0 != 3 && c1 != 3) ? 3 : (c0 != 2 && c1 != 2) ? 2 : 1;
+    const double d1 = pick(dx, x1), d2 = pick(dx, x2);
+    /* the cut on edge k at (a_k, b_k) */
+    double a0 = 0, b1 = 0, b2 = 0, a3 = 0;
+    const bool k0 = edge_cut(P[0][0], P[1][0], E0, d1, a0), k1 = edge_cut(P[0][0], P[0][1], E0, d2, b1);
+    const bool k2 = edge_cut(P[1][0], P[1][1], E0, d2, b2), k3 = edge_cut(P[0][1], P[1][1], E0, d1, a3);
+    const int nc = k0 + k1 + k2 + k3;
     if (nc != 0 && nc != 2 && nc != 4) { w.error = true; return; }
     if (nc == 0) return;
-    bool ambiguous = false;
+    double ca[4], cb[4], oa[2], ob[2];
     if (nc == 4) {
-        ambiguous = true;
+        ca[0] = a0; cb[0] = 0; ca[1] = 0; cb[1] = b1; ca[2] = d1; cb[2] = b2; ca[3] = a3; cb[3] = d2;
         double Emid = 0;
         for (int i = 0; i < 2; i++)
             for (int j = 0; j < 2; j++) Emid += 0.25 * P[i][j];
-        if ((P[0][0] < E0 && Emid < E0) || (P[0][0] > E0 && Emid > E0))
-            for (int i = 0; i < 2; i++) { double t = cuts[1][i]; cuts[1][i] = cuts[2][i]; cuts[2][i] = t; }
+        if ((P[0][0] < E0 && Emid < E0) || (P[0][0] > E0 && Emid > E0)) {
+            const double ta = ca[1], tb = cb[1];
+            ca[1] = ca[2]; cb[1] = cb[2];
+            ca[2] = ta; cb[2] = tb;
+        }
         if ((Emid - E0) < 0) {
-            out[0][0] = out[1][0] = 0.5 * d1;
-            out[0][1] = out[1][1] = 0.5 * d2;
+            oa[0] = oa[1] = 0.5 * d1;
+            ob[0] = ob[1] = 0.5 * d2;
         } else if ((P[0][0] - E0) < 0) {
-            out[0][0] = 0; out[0][1] = 0; out[1][0] = d1; out[1][1] = d2;
+            oa[0] = 0; ob[0] = 0; oa[1] = d1; ob[1] = d2;
         } else {
-            out[0][0] = d1; out[0][1] = 0; out[1][0] = 0; out[1][1] = d2;
+            oa[0] = d1; ob[0] = 0; oa[1] = 0; ob[1] = d2;
         }
     } else {
-        out[0][0] = out[0][1] = out[1][0] = out[1][1] = 0;
+        /* the first and the last cut edge */
+        ca[0] = k0 ? a0 : k1 ? 0 : d1;
+        cb[0] = k0 ? 0 : k1 ? b1 : b2;
+        ca[1] = k3 ? a3 : k2 ? d1 : 0;
+        cb[1] = k3 ? d2 : k2 ? b2 : b1;
+        ca[2] = cb[2] = ca[3] = cb[3] = 0;
+        oa[0] = ob[0] = 0;
         int nout = 0;
         for (int i = 0; i < 2; i++)
             for (int j = 0; j < 2; j++)
-                if (P[i][j] < E0) { out[0][0] += i * d1; out[0][1] += j * d2; nout++; }
-        if (nout > 0)
-            for (int i = 0; i < 2; i++)
-                for (int j = 0; j < 2; j++) out[i][j] = out[i][j] / (double)nout;
+                if (P[i][j] < E0) { oa[0] += i * d1; ob[0] += j * d2; nout++; }
+        if (nout > 0) { oa[0] = oa[0] / (double)nout; ob[0] = ob[0] / (double)nout; }
+        oa[1] = ob[1] = 0;
     }
-    (void)ambiguous;
-    for (int k = 0; k < nc / 2; k++) {
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        if (k == 1 && nc == 2) break;
         if (w.nl >= w.lcap) { w.error = true; return; }
-        int l = w.nl++;
+        const int l = w.nl++;
+#pragma unroll
         for (int e = 0; e < 2; e++) {
-            w.p[l][e][x1] = cuts[2 * k + e][0];
-            w.p[l][e][x2] = cuts[2 * k + e][1];
+            w.p[l][e][x1] = ca[2 * k + e];
+            w.p[l][e][x2] = cb[2 * k + e];
             w.p[l][e][c0] = v0_;
             w.p[l][e][c1] = v1_;
         }
-        w.out[l][x1] = out[k][0];
-        w.out[l][x2] = out[k][1];
+        w.out[l][x1] = oa[k];
+        w.out[l][x2] = ob[k];
         w.out[l][c0] = v0_;
         w.out[l][c1] = v1_;
         w.flip[l] = 0;
@@ -248,14 +259,18 @@ static __device__ const double *poly_centroid(const WorkRef &w, Poly &p)
         return p.cen;
     }
     double up[D] = {0, 0, 0, 0}, down = 0;
+    const int ci = p.const_i;
     for (int i = 0; i < p.nlines; i++) {
         const double *p1 = lstart(w, p.line[i]), *p2 = lend(w, p.line[i]);
         double cm[D], a[D], b[D];
-        for (int j = 0; j < D; j++) cm[j] = (p1[j] + p2[j] + mean[j]) / 3.0;
+        for (int j = 0; j < D; j++) cm[j] = div_rcp(p1[j] + p2[j] + mean[j], 3.0, 1.0 / 3.0);
         for (int j = 0; j < D; j++) { a[j] = p1[j] - mean[j]; b[j] = p2[j] - mean[j]; }
-        double s1 = a[p.x2] * b[p.x3] - a[p.x3] * b[p.x2];
-        double s2 = a[p.x1] * b[p.x3] - a[p.x3] * b[p.x1];
-        double s3 = a[p.x2] * b[p.x1] - a[p.x1] * b[p.x2];
+        /* the components x1 < x2 < x3 other than const_i */
+        const double a1 = ci == 0 ? a[1] : a[0], a2 = ci <= 1 ? a[2] : a[1], a3 = ci <= 2 ? a[3] : a[2];
+        const double b1 = ci == 0 ? b[1] : b[0], b2 = ci <= 1 ? b[2] : b[1], b3 = ci <= 2 ? b[3] : b[2];
+        double s1 = a2 * b3 - a3 * b2;
+        double s2 = a1 * b3 - a3 * b1;
+        double s3 = a2 * b1 - a1 * b2;
         double A = 0.5 * sqrt(s1 * s1 + s2 * s2 + s3 * s3);
         for (int j = 0; j < D; j++) up[j] += cm[j] * A;
         down += A;
@@ -331,9 +346,10 @@ static __device__ int cube_polygons(WorkRef &w, const double cube[2][2][2], int 
             double sq[2][2];
             for (int a = 0; a < 2; a++)
                 for (int b = 0; b < 2; b++)
-                    sq[a][b] = (i == x1) ? cube[j][a][b] : (i == x2) ? cube[a][j][b] : cube[a][b][j];
+                    sq[a][b] = (i == x1) ? (j ? cube[1][a][b] : cube[0][a][b])
+                             : (i == x2) ? (j ? cube[a][1][b] : cube[a][0][b]) : (j ? cube[a][b][1] : cube[a][b][0]);
             int before = w.nl;
-            square_lines(w, sq, const_i, i, const_v, j * dx[i], E0, dx);
+            square_lines(w, sq, const_i, i, const_v, j * pick(dx, i), E0, dx);
             if (w.nl - before == 2) amb++;   /* two lines <=> four cuts: Square::ambiguous */
             if (w.error) return 0;
         }
@@ -363,7 +379,8 @@ __device__ __forceinline__ int cube_line_count(const double cube[2][2][2], int c
             double sq[2][2];
             for (int a = 0; a < 2; a++)
                 for (int b = 0; b < 2; b++)
-                    sq[a][b] = (i == x1) ? cube[j][a][b] : (i == x2) ? cube[a][j][b] : cube[a][b][j];
+                    sq[a][b] = (i == x1) ? (j ? cube[1][a][b] : cube[0][a][b])
+                             : (i == x2) ? (j ? cube[a][1][b] : cube[a][0][b]) : (j ? cube[a][b][1] : cube[a][b][0]);
             const int nc = square_cut_count(sq, E0);
             if (nc != 0 && nc != 2 && nc != 4) err = true;
             n += nc / 2;

@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(128) fo_count3_kernel(const __grid_constant__ 
         const int nlines = __shfl_sync(gmask, incl, 7, 8), at = incl - nl;
         if (nl > 0) {
             cor::WorkRef w{S.p[g], S.out[g], S.flip[g], S.poly[g], at, 0, at + nl, kC3Polys, false};
-            cor::square_lines(w, sq, 0, axis, 0, end * dx[axis], a.eF, dx);
+            cor::square_lines(w, sq, 0, axis, 0, end * cor::pick(dx, axis), a.eF, dx);
             err = err || w.error || w.nl != at + nl;
         }
         bool ambiguous = (__ballot_sync(gmask, nl == 2) & gmask) != 0 || nlines == 6;
@@ -428,7 +428,7 @@ __global__ void __launch_bounds__(128) fo_count3_kernel(const __grid_constant__ 
                     if (r + q < n) {
                         const double *p1 = cor::lstart(w, P.line[r + q]), *p2 = cor::lend(w, P.line[r + q]);
                         double cm[4], d1[4], d2[4];
-                        for (int j = 0; j < 4; j++) cm[j] = (p1[j] + p2[j] + mean[j]) / 3.0;
+                        for (int j = 0; j < 4; j++) cm[j] = div_rcp(p1[j] + p2[j] + mean[j], 3.0, 1.0 / 3.0);
                         for (int j = 0; j < 4; j++) { d1[j] = p1[j] - mean[j]; d2[j] = p2[j] - mean[j]; }
                         const double s1 = d1[2] * d2[3] - d1[3] * d2[2];
                         const double s2 = d1[1] * d2[3] - d1[3] * d2[1];
@@ -655,7 +655,7 @@ __global__ void __launch_bounds__(128, 3) fo_count4_kernel(const __grid_constant
             const int rl = lb - off_l, rp = pb - off_p;
             if (mine && nlc > 0 && !errc) {
                 cor::WorkRef w{S.p, S.out, S.flip, S.poly, rl, rp, rl + nlc, rp + npm, false};
-                const int n = cor::cube_polygons(w, cu, ci, cj * dx[ci], E0, dx, &ambb);
+                const int n = cor::cube_polygons(w, cu, ci, cj * cor::pick(dx, ci), E0, dx, &ambb);
                 if (w.error || n != nlc || w.nl != rl + nlc) errb = true;
                 else {
                     npc = w.np - rp;
