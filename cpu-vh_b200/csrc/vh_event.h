@@ -115,11 +115,13 @@ static inline vh::DevEos dev_eos(const vh_event *ev)
      * leaves every lookup to the plain root solve) */
     auto ranged = [](double x) { return x >= 0x1p-60 && x < 0x1p60; };
     E.direct = 120u << 20;
+    E.ranged = 1;
     if (ev->cfg.eos_kind == VH_EOS_TABLE) {
         unsigned long long b;
         std::memcpy(&b, &E.cs2_third_hi, 8);
         const unsigned hi = (unsigned)(b >> 32), lo = (1023u - 60u) << 20;
-        if (!(E.cs2_third_hi >= 0x1p-60) || !ranged(E.e_spacing) || !(E.e_min == 0 || ranged(E.e_min))) E.direct = 0;
+        E.ranged = ranged(E.e_spacing) && (E.e_min == 0 || ranged(E.e_min));
+        if (!(E.cs2_third_hi >= 0x1p-60) || !E.ranged) E.direct = 0;
         else E.direct = hi - lo < E.direct ? hi - lo : E.direct;
     }
     E.pq.keys = ev->powf.keys;

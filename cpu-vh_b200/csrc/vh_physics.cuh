@@ -26,8 +26,9 @@ struct DevEos {
     double e_min, e_spacing;
     double inv_spacing;       /* RN(1/e_spacing), for div_rcp */
     double cs2_third_hi;      /* eos_cs2 is exactly 1/3 for e <= this (HostEos::cs2_third_bound) */
-    unsigned direct;          /* flow_pair's root solve: 2^-60 <= e with a high word less than `direct` above that
+    unsigned direct;          /* flow_pair's root solve: 2^-60 <= |e| with a high word less than `direct` above that
                                  of 2^-60 is below min(2^60, cs2_third_hi); 0: not for this table */
+    int ranged;               /* the table's e_min and e_spacing lie where eos_interp_direct is exact */
     PowfTab pq;               /* host-exact powf(x, 0.25) */
     const int *stop;          /* the event's device error code (or null): see e_bisect_table */
 };
@@ -345,9 +346,11 @@ __device__ __forceinline__ bool energy_direct(const DevEos &E, const double (&M0
 #pragma unroll
             for (int s = 0; s < N; ++s) {
                 const double x = e0[s];
-                bool fine = (unsigned)__double2hiint(x) - ((1023u - 60u) << 20) < E.direct && rcp_ok(x);
-                const double pp = eos_interp_direct<MIXED>(E, x, E.p_tb);     /* above the floor */
-                fine = fine && within<-49, 60>(pp);
+                /* (an iterate below zero, on its way down a steep gradient, is in
+                 * range too: its p is the floor, 2^-49.8) */
+                bool fine = ((unsigned)__double2hiint(x) & 0x7fffffffu) - ((1023u - 60u) << 20) < E.direct && rcp_ok(x);
+                const double pp = floor15(eos_interp_direct<MIXED>(E, x, E.p_tb));
+                fine = fine && within<-50, 60>(pp);
                 const double yx = rcp_rn(x);
                 const double cst2 = div_rn(pp, x, yx);
                 const double A = M0[s] * (1.0 - cst2) + Pi[s];

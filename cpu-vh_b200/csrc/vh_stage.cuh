@@ -725,7 +725,7 @@ template <int NQ, int EOS>
 __device__ __forceinline__ bool source_direct(const StageArgs &A, long long s, double *__restrict__ acc)
 {
     DirectQuot<> dv;
-    dv.ok = A.eos.direct && in_range(A.t) && in_range(A.dx) && in_range(A.dy) && in_range(A.dz) && in_range(A.etabar) &&
+    dv.ok = A.eos.ranged && in_range(A.t) && in_range(A.dx) && in_range(A.dy) && in_range(A.dz) && in_range(A.etabar) &&
             in_range(2 * A.t);
     source_terms<NQ, EOS>(dv, A, s, acc);
     unsigned top = 0;
