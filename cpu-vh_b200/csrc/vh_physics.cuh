@@ -225,6 +225,21 @@ __device__ __forceinline__ double e_newton_table_body(const DevEos &E, double eP
     return e_bisect_table(E, ePrev, M0, M, Pi);
 }
 
+/* the same from iterate e0 of iteration j0 on, out of line: a solve that is
+ * still going after the few iterations it usually takes */
+static __device__ __noinline__ double e_newton_rest(const DevEos &E, double e0, int j0, double ePrev, double M0, double M,
+                                                    double Pi, bool &bad)
+{
+    for (int j = j0; j < 10000; ++j) {
+        bool nan_step, conv;
+        double e = e_newton_iter(E, e0, M0, M, Pi, nan_step, conv);
+        if (nan_step) { bad = true; return ePrev; }
+        if (conv) return e;
+        e0 = e;
+    }
+    return e_bisect_table(E, ePrev, M0, M, Pi);
+}
+
 /* The root solve as a call (one copy of the loop for a long kernel whose
  * instruction footprint matters) or inlined (short phase kernels). */
 static __device__ __noinline__ double e_newton_table(const DevEos &E, double ePrev, double M0, double M, double Pi, bool &bad)
@@ -309,8 +324,12 @@ __device__ __forceinline__ float root32(float x)
 }
 
 /* the energy density of N states (e_from_conserved, or infer's closed form
- * below ePrev = 0.1); M = M1^2 + M2^2 + t^2 M3^2 */
-template <int EOS, int N, bool MIXED>
+ * below ePrev = 0.1); M = M1^2 + M2^2 + t^2 M3^2.  REST: a solve still going
+ * after 8 iterations (one state in a steep gradient of a coarse lattice) ends
+ * out of line, alone; the call costs the line-piece kernels registers (mixed
+ * 131x131x61 4 %), so only the fused stage, whose time is its slowest thread,
+ * takes it (21x21x9: 100 -> 84 us per step, mixed 91 -> 77) */
+template <int EOS, int N, bool MIXED, bool REST = false>
 __device__ __forceinline__ bool energy_direct(const DevEos &E, const double (&M0)[N], const double (&M)[N],
                                               const double (&Pi)[N], double ePrev, double (&ef)[N])
 {
@@ -341,6 +360,15 @@ __device__ __forceinline__ bool energy_direct(const DevEos &E, const double (&M0
         }
         const double cs2 = 1. / 3.;
         for (int j = 0; ok; ++j) {
+            if (REST && j == 8) {
+                /* few lanes are left, and of those mostly one state */
+                bool bad = false;
+#pragma unroll
+                for (int s = 0; s < N; ++s)
+                    if (!done[s]) ef[s] = e_newton_rest(E, e0[s], j, ePrev, M0[s], M[s], Pi[s], bad);
+                ok = !bad;
+                break;
+            }
             if (j == 100) { ok = false; break; }
             bool all = true;
 #pragma unroll
@@ -403,7 +431,7 @@ __device__ __forceinline__ bool flow_direct(const DevEos &E, double M0, double P
     return ok;
 }
 
-template <int EOS, bool MIXED = false>
+template <int EOS, bool MIXED = false, bool REST = false>
 __device__ __forceinline__ bool flow_pair(const DevEos &E, double t, const double (&M0)[2], const double (&M1)[2],
                                           const double (&M2)[2], const double (&M3)[2], const double (&Pi)[2], int dir,
                                           double ePrev, Flow (&out)[2])
@@ -411,7 +439,7 @@ __device__ __forceinline__ bool flow_pair(const DevEos &E, double t, const doubl
     double M[2], ef[2];
 #pragma unroll
     for (int s = 0; s < 2; ++s) M[s] = M1[s] * M1[s] + M2[s] * M2[s] + t * t * M3[s] * M3[s];
-    bool ok = energy_direct<EOS, 2, MIXED>(E, M0, M, Pi, ePrev, ef);
+    bool ok = energy_direct<EOS, 2, MIXED, REST>(E, M0, M, Pi, ePrev, ef);
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
         double p, ut, yu, E2;

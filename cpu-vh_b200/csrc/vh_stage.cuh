@@ -1007,7 +1007,7 @@ __device__ __forceinline__ void extrapolate_m(const double *__restrict__ qn, lon
  * so that its rounding does not hang on how the compiler contracts the sum in
  * one kernel or another; LFIRST: sL qL is the product that is added unrounded
  * (the face a cell evaluates for itself across the e <= 0.1 branch). */
-template <int NQ, int EOS, bool LFIRST = false>
+template <int NQ, int EOS, bool LFIRST = false, bool REST = false>
 __device__ __forceinline__ void face_flux_m(const StageArgs &A, long long b, long long st, int dir, bool fwd,
                                             double ePrev, double *__restrict__ r, bool &bad)
 {
@@ -1026,7 +1026,7 @@ __device__ __forceinline__ void face_flux_m(const StageArgs &A, long long b, lon
 #pragma unroll
     for (int c = 0; c < 8; ++c) direct = direct && half_state_ranged(qRs[c]) && half_state_ranged(qLs[c]);
     Flow F[2];
-    direct = flow_pair<EOS, true>(A.eos, A.t, M0, M1, M2, M3, Pi, dir, ePrev, F) && direct;
+    direct = flow_pair<EOS, true, REST>(A.eos, A.t, M0, M1, M2, M3, Pi, dir, ePrev, F) && direct;
     float sR = (float)F[0].v / (float)F[0].ut, sL = (float)F[1].v / (float)F[1].ut;
     if (!direct) {
         flow_pair_plain<EOS>(A.eos, A.t, M0, M1, M2, M3, Pi, dir, ePrev, F, bad);
@@ -1388,7 +1388,7 @@ __device__ __forceinline__ bool face_direct(const StageArgs &A, long long b, lon
     const double M2[2] = {qR[2] - qR[6], qL[2] - qL[6]}, M3[2] = {qR[3] - qR[7], qL[3] - qL[7]};
     const double Pi[2] = {(NQ == 15) ? qR[NQ - 1] : 0.0, (NQ == 15) ? qL[NQ - 1] : 0.0};
     Flow F[2];
-    ok = flow_pair<EOS>(A.eos, A.t, M0, M1, M2, M3, Pi, dir, ePrev, F) && ok;
+    ok = flow_pair<EOS, false, true>(A.eos, A.t, M0, M1, M2, M3, Pi, dir, ePrev, F) && ok;
     const double a = fmax(fabs(div_rn(F[1].v, F[1].ut, F[1].y)), fabs(div_rn(F[0].v, F[0].ut, F[0].y)));
 #pragma unroll
     for (int n = 0; n < NQ; ++n) {
@@ -1438,7 +1438,7 @@ __device__ __forceinline__ void stage_faces_cell(const StageArgs &A, int i, int 
         if constexpr (MIXED) {
 #pragma unroll
             for (int n = 0; n < NQ; ++n) r[n] = -0.0;
-            face_flux_m<NQ, EOS>(A, fwd ? s : s - st, st, dir, fwd, ePrev, r, bad);
+            face_flux_m<NQ, EOS, false, true>(A, fwd ? s : s - st, st, dir, fwd, ePrev, r, bad);
 #pragma unroll
             for (int n = 0; n < NQ; ++n) col[n * TX] = r[n];
         } else if (face_direct<NQ, EOS>(A, fwd ? s : s - st, st, dir, fwd, ePrev, r)) {
