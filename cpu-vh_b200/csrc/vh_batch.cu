@@ -160,7 +160,8 @@ static int resident_blocks(BatchKernel k)
     auto it = cache.find(k);
     if (it != cache.end()) return it->second;
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, 128, 0) != cudaSuccess || nb < 1) nb = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, 128, 0) != cudaSuccess) cudaGetLastError();
+    if (nb < 1) nb = 1;
     cache[k] = nb;
     return nb;
 }
@@ -227,9 +228,7 @@ int bfail(int code, const std::string &msg) { return vh::set_error(code, msg); }
 #define BTRY(x)                                                                                        \
     do {                                                                                               \
         cudaError_t e__ = (x);                                                                         \
-        if (e__ != cudaSuccess)                                                                        \
-            return bfail(e__ == cudaErrorMemoryAllocation ? VH_ERR_NOMEM : VH_ERR_CUDA,                \
-                         std::string(#x) + ": " + cudaGetErrorString(e__));                            \
+        if (e__ != cudaSuccess) return vh::cuda_error(#x, e__);                                        \
     } while (0)
 
 int build_tiles(vh_batch *b, int tx)
@@ -399,7 +398,7 @@ vh::StageMarks *next_marks(vh_batch *b)
     if (b->marks_used == b->marks.size()) {
         vh::StageMarks m{};
         for (cudaEvent_t &e : m.ev)
-            if (cudaEventCreate(&e) != cudaSuccess) return nullptr;
+            if (cudaEventCreate(&e) != cudaSuccess) { cudaGetLastError(); return nullptr; }
         b->marks.push_back(m);
     }
     return &b->marks[b->marks_used++];
@@ -646,7 +645,7 @@ int ensure_graph(vh_batch *b)
     launch_stage(b, 1, b->tune, nullptr);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(b->stream, &g);
-    if (e != cudaSuccess) return bfail(VH_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) { vh::cuda_error("graph capture", e); return VH_ERR_CUDA; }
     b->graph = g;
     BTRY(cudaGraphInstantiate(&b->exec, g, 0));
     return VH_OK;
@@ -672,7 +671,7 @@ int vh_batch_create(vh_event *const *events, int n_events, vh_batch **out)
     *out = nullptr;
     vh_batch *b = new vh_batch;
     int rc = VH_OK;
-#define CTRY(x) do { cudaError_t e__ = (x); if (e__ != cudaSuccess) { rc = bfail(e__ == cudaErrorMemoryAllocation ? VH_ERR_NOMEM : VH_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e__)); vh_batch_destroy(b); return rc; } } while (0)
+#define CTRY(x) do { cudaError_t e__ = (x); if (e__ != cudaSuccess) { rc = vh::cuda_error(#x, e__); vh_batch_destroy(b); return rc; } } while (0)
     for (int i = 0; i < n_events; ++i) {
         vh_event *ev = events[i];
         if (!ev) { vh_batch_destroy(b); return bfail(VH_ERR_ARG, "null member"); }

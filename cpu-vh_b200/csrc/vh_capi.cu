@@ -30,11 +30,18 @@ static int fail(int code, const std::string &msg)
 }
 
 int vh::set_error(int code, const std::string &msg) { return fail(code, msg); }
+/* a failed call's message and status.  The runtime keeps the error of a failed
+ * call for cudaGetLastError(), which is how launches are checked: it is taken
+ * away here, so that the next call does not report it again as its own */
+int vh::cuda_error(const char *what, cudaError_t e)
+{
+    (void)cudaGetLastError();
+    return fail(e == cudaErrorMemoryAllocation ? VH_ERR_NOMEM : VH_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+}
 #define CUDA_TRY(x)                                                                                   \
     do {                                                                                              \
         cudaError_t e__ = (x);                                                                        \
-        if (e__ != cudaSuccess) return fail(e__ == cudaErrorMemoryAllocation ? VH_ERR_NOMEM : VH_ERR_CUDA, \
-                                            std::string(#x) + ": " + cudaGetErrorString(e__));        \
+        if (e__ != cudaSuccess) return vh::cuda_error(#x, e__);                                       \
     } while (0)
 
 namespace {
@@ -222,7 +229,7 @@ int vh_event_create(const vh_config *cfg, const double *eos_rows, int eos_nrows,
     ev->e_reg = ev->heos.energy_of_T(cfg->T_reg_GeV / vh::kHbarc);
     ev->e_fo = ev->heos.energy_of_T(cfg->T_freezeout_GeV / vh::kHbarc);
     int rc;
-#define TRY(x) do { cudaError_t e__ = (x); if (e__ != cudaSuccess) { rc = fail(e__ == cudaErrorMemoryAllocation ? VH_ERR_NOMEM : VH_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e__)); vh_event_destroy(ev); return rc; } } while (0)
+#define TRY(x) do { cudaError_t e__ = (x); if (e__ != cudaSuccess) { rc = vh::cuda_error(#x, e__); vh_event_destroy(ev); return rc; } } while (0)
     TRY(cudaGetDevice(&ev->device));
     TRY(cudaStreamCreateWithFlags(&ev->stream, cudaStreamNonBlocking));
     pool_live(ev->device, 1);
@@ -366,7 +373,7 @@ static vh::StageMarks *next_marks(vh_event *ev)
     if (ev->marks_used == ev->marks.size()) {
         vh::StageMarks m{};
         for (cudaEvent_t &e : m.ev)
-            if (cudaEventCreate(&e) != cudaSuccess) return nullptr;
+            if (cudaEventCreate(&e) != cudaSuccess) { cudaGetLastError(); return nullptr; }
         ev->marks.push_back(m);
     }
     return &ev->marks[ev->marks_used++];
@@ -735,7 +742,7 @@ int vh_device_math_check(int which, const double *a, const double *b, int n, dou
     }
     if (e == cudaSuccess) e = cudaMemcpy(out, d + 2 * (size_t)n, B, cudaMemcpyDeviceToHost);
     cudaFree(d);
-    if (e != cudaSuccess) return fail(VH_ERR_CUDA, std::string("vh_device_math_check: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) { vh::cuda_error("vh_device_math_check", e); return VH_ERR_CUDA; }
     return VH_OK;
 }
 
@@ -756,7 +763,7 @@ int vh_device_round_check(int which, const double *a, const double *b, int n, do
     }
     if (e == cudaSuccess) e = cudaMemcpy(out, d + 2 * (size_t)n, 2 * B, cudaMemcpyDeviceToHost);
     cudaFree(d);
-    if (e != cudaSuccess) return fail(VH_ERR_CUDA, std::string("vh_device_round_check: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) { vh::cuda_error("vh_device_round_check", e); return VH_ERR_CUDA; }
     return VH_OK;
 }
 
@@ -776,7 +783,7 @@ int vh_cornelius_surfaces(int dim, const double *cubes, int n_cubes, double valu
     int rc = VH_OK;
     std::vector<double> slots;
     std::vector<int> cnt;
-#define GO(x) do { cudaError_t e__ = (x); if (e__ != cudaSuccess) { rc = fail(VH_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e__)); goto done; } } while (0)
+#define GO(x) do { cudaError_t e__ = (x); if (e__ != cudaSuccess) { vh::cuda_error(#x, e__); rc = VH_ERR_CUDA; goto done; } } while (0)
     GO(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     GO(cudaMalloc(&d_cubes, (size_t)n_cubes * per * sizeof(double)));
     GO(cudaMalloc(&d_slots, slot_doubles * sizeof(double)));

@@ -137,6 +137,9 @@ static inline vh::DevEos dev_eos(const vh_event *ev)
 namespace vh {
 /* the step-independent part of a stage's arguments (pointers and times unset) */
 StageArgs stage_args_base(const vh_event *ev);
+/* records a failed runtime call as the thread's vh_last_error(), clears the
+ * runtime's own record of it and returns VH_ERR_NOMEM or VH_ERR_CUDA */
+int cuda_error(const char *what, cudaError_t e);
 } // namespace vh
 
 #endif

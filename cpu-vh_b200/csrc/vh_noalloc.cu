@@ -161,8 +161,10 @@ extern "C" int vh_cornelius_surfaces_noalloc(int dim, const double *d_cubes, int
     cudaError_t rc = cudaGetDevice(&dev);
     int *base = nullptr;
     if (rc == cudaSuccess) rc = vh::scratch_address(dev, &base);
-    if (rc != cudaSuccess)
+    if (rc != cudaSuccess) {
+        (void)cudaGetLastError();   /* not to be taken for a launch's by the next call */
         return vh::set_error(VH_ERR_CUDA, std::string("vh_cornelius_surfaces_noalloc: ") + cudaGetErrorString(rc));
+    }
     cudaStream_t st = (cudaStream_t)stream;
     const double d3 = dim == 4 ? dx[3] : 0.0;
     const unsigned grid = (unsigned)((n_cubes + 127) / 128);

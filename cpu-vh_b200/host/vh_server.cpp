@@ -459,7 +459,7 @@ int vh_server_create(const vh_server_config *cfg, const double *eos_rows, int eo
     if (eos_rows && eos_nrows > 0) S->eos_rows.assign(eos_rows, eos_rows + 4 * (size_t)eos_nrows);
     cudaGetDevice(&S->device);
     size_t fr = 0, tot = 0;
-    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) { delete S; return vh::set_error(VH_ERR_CUDA, "cudaMemGetInfo"); }
+    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) { cudaGetLastError(); delete S; return vh::set_error(VH_ERR_CUDA, "cudaMemGetInfo"); }
     S->budget = (size_t)(c.hbm_fraction * (double)fr);
     S->st.budget_bytes = S->budget;
     S->t0 = Clock::now();
