@@ -676,9 +676,11 @@ int vh_event_freezeout_finish(vh_event *ev, int *n_elements, int *n_above)
         /* not enough room: a buffer with room to grow, and the emit step
          * again from the offsets the block left in the scratch */
         ev_free(ev, ev->fo_elems);
-        ev->fo_elems = nullptr;
-        ev->fo_cap = total + total / 2 + 1024;
-        CUDA_TRY(ev_alloc(ev, &ev->fo_elems, (size_t)ev->fo_cap * VH_FO_COLUMNS * sizeof(double)));
+        ev->fo_elems = nullptr;       /* where the allocation fails: no rows to read, and the next block asks again */
+        ev->fo_cap = 0;
+        const int cap = total + total / 2 + 1024;
+        CUDA_TRY(ev_alloc(ev, &ev->fo_elems, (size_t)cap * VH_FO_COLUMNS * sizeof(double)));
+        ev->fo_cap = cap;
         vh::FoArgs a;
         fo_args(ev, a);
         vh::launch_freezeout_emit(a, ev->stream);
@@ -706,6 +708,8 @@ int vh_event_fetch_surface(vh_event *ev, double *host_out, int cap_elements, int
     if (ev->fo_count > cap_elements) return fail(VH_ERR_CAPACITY, "surface buffer too small");
     if (ev->fo_count == 0) return VH_OK;
     if (!host_out) return fail(VH_ERR_ARG, "null output");
+    /* the pinned rows are those of fo_elems' block and end with it */
+    if (!ev->fo_elems) return fail(VH_ERR_STATE, "the surface was lost when its buffer could not grow");
     if (ev->fo_count <= vh::kFoHostElems && !ev->fo_pending) {
         std::memcpy(host_out, ev->fo_host, (size_t)ev->fo_count * VH_FO_COLUMNS * sizeof(double));
         return VH_OK;

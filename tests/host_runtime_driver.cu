@@ -266,6 +266,27 @@ void error_cleared()
     vh_event_destroy(ev);
 }
 
+/* the element buffer cannot grow: neither that block nor the one before it
+ * can be read any more, and later blocks are whole again */
+void regrow_failure()
+{
+    setenv("VH_FO_INITIAL_CAP", "4", 1);
+    vh_event *ev = make(9, 8, 1);
+    good_block(ev, 3, 1);
+    block_total = 10; block_value = 2;
+    expect(vh_event_freezeout_launch(ev) == VH_OK, "launch");
+    counting = true; counted = 0; fail_at = 0;
+    expect(vh_event_freezeout_finish(ev, nullptr, nullptr) != VH_OK, "the failed growth is reported");
+    counting = false;
+    std::vector<double> rows(20 * VH_FO_COLUMNS, -1.0);
+    int n = 0;
+    expect(vh_event_fetch_surface(ev, rows.data(), 20, &n) != VH_OK, "lost rows are not handed out");
+    good_block(ev, 2, 3);
+    good_block(ev, 12, 4);
+    expect(!null_store, "kernels get every buffer");
+    vh_event_destroy(ev);
+}
+
 void step(vh_event *ev, const char *what) { expect(vh_event_step(ev, 2) == VH_OK, what); }
 
 } // namespace
@@ -273,7 +294,8 @@ void step(vh_event *ev, const char *what) { expect(vh_event_step(ev, 2) == VH_OK
 int main(int argc, char **argv)
 {
     const std::map<std::string, void (*)()> all = {
-        {"error_cleared", error_cleared}};
+        {"error_cleared", error_cleared},
+        {"regrow_failure", regrow_failure}};
     auto it = argc > 1 ? all.find(argv[1]) : all.end();
     if (it == all.end()) return 2;
     it->second();
