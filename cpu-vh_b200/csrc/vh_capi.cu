@@ -623,38 +623,60 @@ static void fo_args(vh_event *ev, vh::FoArgs &a)
     a.slot_cap = ev->fo_slot_cap;
 }
 
+/* what an event's first block sets up, and its undoing */
+static void freezeout_drop(vh_event *ev)
+{
+    for (double **p : {&ev->fo_slabs, &ev->fo_elems, &ev->fo_slots}) { ev_free(ev, *p); *p = nullptr; }
+    ev_free(ev, ev->fo_scratch);
+    if (ev->fo_hdr) cudaFreeHost(ev->fo_hdr);
+    if (ev->fo_host) cudaFreeHost(ev->fo_host);
+    if (ev->fo_done) cudaEventDestroy(ev->fo_done);
+    ev->fo_scratch = nullptr;
+    ev->fo_hdr = nullptr;
+    ev->fo_host = nullptr;
+    ev->fo_done = nullptr;
+    ev->fo_cap = ev->fo_slot_cap = 0;
+    ev->fo_ready = false;
+}
+
+static int freezeout_setup(vh_event *ev)
+{
+    const vh_config &c = ev->cfg;
+    const size_t N = (size_t)ev->N;
+    CUDA_TRY(ev_alloc(ev, &ev->fo_slabs, 2 * 11 * N * sizeof(double)));
+    CUDA_TRY(cudaMemsetAsync(ev->fo_slabs, 0, 2 * 11 * N * sizeof(double), ev->stream));
+    ev->fo_scratch_ints = vh::freezeout_scratch_ints(c.nx, c.ny, c.nz);
+    CUDA_TRY(ev_alloc(ev, &ev->fo_scratch, ev->fo_scratch_ints * sizeof(int)));
+    CUDA_TRY(cudaMemsetAsync(ev->fo_scratch + ev->fo_scratch_ints - vh::kFoHeaderInts, 0, vh::kFoHeaderInts * sizeof(int),
+                             ev->stream));
+    CUDA_TRY(cudaMallocHost(&ev->fo_hdr, 2 * sizeof(int)));
+    CUDA_TRY(cudaMallocHost(&ev->fo_host, (size_t)vh::kFoHostElems * VH_FO_COLUMNS * sizeof(double)));
+    CUDA_TRY(cudaEventCreateWithFlags(&ev->fo_done, cudaEventDisableTiming));
+    /* a first element buffer sized for a surface crossing the lattice
+     * (twice its cross sections in 3+1D, eight times its edges in 2+1D),
+     * so that blocks seldom overflow it; VH_FO_INITIAL_CAP overrides the
+     * size (tests of the overflow path) */
+    const long long nx = c.nx, ny = c.ny, nz = c.nz;
+    long long cap = (nz > 1 ? 2 * (nx * ny + ny * nz + nx * nz) : 8 * (nx + ny)) + 1024;
+    if (const char *env = getenv("VH_FO_INITIAL_CAP")) cap = std::max(1LL, atoll(env));
+    ev->fo_cap = (int)std::min<long long>(cap, 1LL << 28);
+    CUDA_TRY(ev_alloc(ev, &ev->fo_elems, (size_t)ev->fo_cap * VH_FO_COLUMNS * sizeof(double)));
+    /* element slots for as many crossed cubes as the first buffer has
+     * elements (a cube beyond them runs Cornelius again in the emit step) */
+    ev->fo_slot_cap = ev->fo_cap;
+    CUDA_TRY(ev_alloc(ev, &ev->fo_slots, (size_t)ev->fo_slot_cap * vh::kFoSlotDoubles * sizeof(double)));
+    ev->fo_ready = true;
+    return VH_OK;
+}
+
 int vh_event_freezeout_launch(vh_event *ev)
 {
     if (!ev) return fail(VH_ERR_ARG, "null event");
     if (!ev->initialised) return fail(VH_ERR_STATE, "freezeout before vh_event_set_initial");
     if (ev->fo_pending) return fail(VH_ERR_STATE, "a freezeout block is already pending");
-    const vh_config &c = ev->cfg;
-    const size_t N = (size_t)ev->N;
-    if (!ev->fo_slabs) {
-        CUDA_TRY(ev_alloc(ev, &ev->fo_slabs, 2 * 11 * N * sizeof(double)));
-        CUDA_TRY(cudaMemsetAsync(ev->fo_slabs, 0, 2 * 11 * N * sizeof(double), ev->stream));
-        ev->fo_scratch_ints = vh::freezeout_scratch_ints(c.nx, c.ny, c.nz);
-        CUDA_TRY(ev_alloc(ev, &ev->fo_scratch, ev->fo_scratch_ints * sizeof(int)));
-        CUDA_TRY(cudaMemsetAsync(ev->fo_scratch + ev->fo_scratch_ints - vh::kFoHeaderInts, 0, vh::kFoHeaderInts * sizeof(int),
-                                 ev->stream));
-        CUDA_TRY(cudaMallocHost(&ev->fo_hdr, 2 * sizeof(int)));
-        CUDA_TRY(cudaMallocHost(&ev->fo_host, (size_t)vh::kFoHostElems * VH_FO_COLUMNS * sizeof(double)));
-        CUDA_TRY(cudaEventCreateWithFlags(&ev->fo_done, cudaEventDisableTiming));
-        /* a first element buffer sized for a surface crossing the lattice
-         * (twice its cross sections in 3+1D, eight times its edges in 2+1D),
-         * so that blocks seldom overflow it; VH_FO_INITIAL_CAP overrides the
-         * size (tests of the overflow path) */
-        if (!ev->fo_elems) {
-            const long long nx = c.nx, ny = c.ny, nz = c.nz;
-            long long cap = (nz > 1 ? 2 * (nx * ny + ny * nz + nx * nz) : 8 * (nx + ny)) + 1024;
-            if (const char *env = getenv("VH_FO_INITIAL_CAP")) cap = std::max(1LL, atoll(env));
-            ev->fo_cap = (int)std::min<long long>(cap, 1LL << 28);
-            CUDA_TRY(ev_alloc(ev, &ev->fo_elems, (size_t)ev->fo_cap * VH_FO_COLUMNS * sizeof(double)));
-            /* element slots for as many crossed cubes as the first buffer has
-             * elements (a cube beyond them runs Cornelius again in the emit step) */
-            ev->fo_slot_cap = ev->fo_cap;
-            CUDA_TRY(ev_alloc(ev, &ev->fo_slots, (size_t)ev->fo_slot_cap * vh::kFoSlotDoubles * sizeof(double)));
-        }
+    if (!ev->fo_ready) {
+        const int rc = freezeout_setup(ev);
+        if (rc != VH_OK) { freezeout_drop(ev); return rc; }
     }
     vh::FoArgs a;
     fo_args(ev, a);

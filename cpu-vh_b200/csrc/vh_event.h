@@ -62,6 +62,7 @@ struct vh_event {
     double t = 0;
     bool initialised = false;
     /* freezeout */
+    bool fo_ready = false;                /* everything a block needs is allocated and cleared */
     double *fo_slabs = nullptr;           /* 2 x 11 x N */
     int fo_prev = 0;                      /* which half is the previous slab */
     int *fo_scratch = nullptr;

@@ -266,6 +266,33 @@ void error_cleared()
     vh_event_destroy(ev);
 }
 
+/* a first block whose set-up fails at its k-th step launches nothing and
+ * leaves nothing allocated; the next call sets up again */
+void setup_rollback()
+{
+    for (int k = 0; k < 64; ++k) {
+        vh_event *ev = make(9, 8, 1);
+        const size_t before = live.size();
+        const int l0 = launches;
+        counting = true; counted = 0; fail_at = k;
+        block_total = 3; block_value = 7;
+        const int rc = vh_event_freezeout(ev, nullptr, nullptr);
+        counting = false;
+        if (rc == VH_OK) {
+            expect(k >= 8, "every step of the set-up was failed once");
+            expect(counted <= k, "a failed step was reported");
+            vh_event_destroy(ev);
+            break;
+        }
+        expect(launches == l0, "no kernel after a failed set-up");
+        expect(live.size() == before, "a failed set-up gives its memory back");
+        good_block(ev, 5, k + 1);
+        expect(!null_store, "kernels get every buffer");
+        expect(!list_overrun, "the crossed-cube counter starts at zero");
+        vh_event_destroy(ev);
+    }
+}
+
 /* the element buffer cannot grow: neither that block nor the one before it
  * can be read any more, and later blocks are whole again */
 void regrow_failure()
@@ -295,7 +322,7 @@ int main(int argc, char **argv)
 {
     const std::map<std::string, void (*)()> all = {
         {"error_cleared", error_cleared},
-        {"regrow_failure", regrow_failure}};
+        {"setup_rollback", setup_rollback}, {"regrow_failure", regrow_failure}};
     auto it = argc > 1 ? all.find(argv[1]) : all.end();
     if (it == all.end()) return 2;
     it->second();
