@@ -639,6 +639,14 @@ static void freezeout_drop(vh_event *ev)
     ev->fo_ready = false;
 }
 
+/* the scratch header, zero before a block: the open step counts the crossed
+ * cubes in it and appends to a list by that count */
+static cudaError_t freezeout_clear_header(vh_event *ev)
+{
+    return cudaMemsetAsync(ev->fo_scratch + ev->fo_scratch_ints - vh::kFoHeaderInts, 0, vh::kFoHeaderInts * sizeof(int),
+                           ev->stream);
+}
+
 static int freezeout_setup(vh_event *ev)
 {
     const vh_config &c = ev->cfg;
@@ -647,8 +655,7 @@ static int freezeout_setup(vh_event *ev)
     CUDA_TRY(cudaMemsetAsync(ev->fo_slabs, 0, 2 * 11 * N * sizeof(double), ev->stream));
     ev->fo_scratch_ints = vh::freezeout_scratch_ints(c.nx, c.ny, c.nz);
     CUDA_TRY(ev_alloc(ev, &ev->fo_scratch, ev->fo_scratch_ints * sizeof(int)));
-    CUDA_TRY(cudaMemsetAsync(ev->fo_scratch + ev->fo_scratch_ints - vh::kFoHeaderInts, 0, vh::kFoHeaderInts * sizeof(int),
-                             ev->stream));
+    CUDA_TRY(freezeout_clear_header(ev));
     CUDA_TRY(cudaMallocHost(&ev->fo_hdr, 2 * sizeof(int)));
     CUDA_TRY(cudaMallocHost(&ev->fo_host, (size_t)vh::kFoHostElems * VH_FO_COLUMNS * sizeof(double)));
     CUDA_TRY(cudaEventCreateWithFlags(&ev->fo_done, cudaEventDisableTiming));
@@ -680,8 +687,12 @@ int vh_event_freezeout_launch(vh_event *ev)
     }
     vh::FoArgs a;
     fo_args(ev, a);
-    vh::launch_freezeout(a, ev->stream);
-    CUDA_TRY(cudaGetLastError());
+    /* a block's own offsets step clears the header for the next; where the
+     * chain of kernels did not get that far, it is cleared here */
+    if (ev->fo_broken) CUDA_TRY(freezeout_clear_header(ev));
+    ev->fo_broken = true;
+    CUDA_TRY(vh::launch_freezeout(a, ev->stream));
+    ev->fo_broken = false;
     CUDA_TRY(cudaEventRecord(ev->fo_done, ev->stream));
     ev->fo_pending = true;
     return VH_OK;
@@ -705,8 +716,7 @@ int vh_event_freezeout_finish(vh_event *ev, int *n_elements, int *n_above)
         ev->fo_cap = cap;
         vh::FoArgs a;
         fo_args(ev, a);
-        vh::launch_freezeout_emit(a, ev->stream);
-        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(vh::launch_freezeout_emit(a, ev->stream));
         CUDA_TRY(cudaStreamSynchronize(ev->stream));
     }
     ev->fo_prev = 1 - ev->fo_prev;

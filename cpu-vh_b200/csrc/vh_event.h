@@ -76,6 +76,7 @@ struct vh_event {
     int *fo_hdr = nullptr;                /* pinned: n_above, n_total of the last block */
     cudaEvent_t fo_done = nullptr;
     bool fo_pending = false;              /* launched, not yet finished */
+    bool fo_broken = false;               /* a block's chain of kernels was not launched to its end */
     /* thermal vorticity (vh_event_vorticity): 6 w planes then 4 beta planes */
     double *vort = nullptr;
     bool vort_on = false;

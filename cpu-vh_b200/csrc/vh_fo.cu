@@ -757,7 +757,7 @@ __global__ void __launch_bounds__(128, 3) fo_count4_kernel(const __grid_constant
 }
 
 template <typename... P, typename... X>
-static void launch_dep(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, const X &...x)
+static cudaError_t launch_dep(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, const X &...x)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
@@ -769,10 +769,10 @@ static void launch_dep(void (*kernel)(P...), unsigned grid, unsigned block, size
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, x...);
+    return cudaLaunchKernelEx(&cfg, kernel, x...);
 }
 
-static void launch_count4(const FoArgs &a, FoScratch sc, cudaStream_t st)
+static cudaError_t launch_count4(const FoArgs &a, FoScratch sc, cudaStream_t st)
 {
     static int blocks = [] {
         int dev = 0, sms = 148;
@@ -785,7 +785,7 @@ static void launch_count4(const FoArgs &a, FoScratch sc, cudaStream_t st)
     }();
     const long long need = ((long long)sc.nc + kG4 - 1) / kG4;
     const unsigned grid = (unsigned)(need < blocks ? (need > 0 ? need : 1) : blocks);
-    launch_dep(fo_count4_kernel, grid, 128, sizeof(Count4Shared), st, a, sc);
+    return launch_dep(fo_count4_kernel, grid, 128, sizeof(Count4Shared), st, a, sc);
 }
 
 /* FreezeOut.cpp:40-55 */
@@ -950,26 +950,30 @@ __global__ void __launch_bounds__(128) fo_emit_kernel(const __grid_constant__ Fo
     }
 }
 
-void launch_freezeout(const FoArgs &a, cudaStream_t st)
+/* stops at the first kernel that does not launch: the later ones read what it writes */
+cudaError_t launch_freezeout(const FoArgs &a, cudaStream_t st)
 {
     const FoScratch sc = carve(a);
     const unsigned N = (unsigned)a.nx * a.ny * a.nz;
-    launch_dep(fo_open_kernel, (N + 255) / 256, 256, 0, st, a, sc);
-    if (a.nz > 1) launch_count4(a, sc, st);
-    else launch_dep(fo_count3_kernel, (unsigned)std::min((sc.nc + kG3 - 1) / kG3, 148 * 8), 128, 0, st, a, sc);
-    launch_dep(fo_offsets_kernel, (unsigned)sc.nb, kScanThreads, 0, st, sc, a.host_hdr);
-    launch_freezeout_emit(a, st);
+    cudaError_t e = launch_dep(fo_open_kernel, (N + 255) / 256, 256, 0, st, a, sc);
+    if (e != cudaSuccess) return e;
+    if (a.nz > 1) e = launch_count4(a, sc, st);
+    else e = launch_dep(fo_count3_kernel, (unsigned)std::min((sc.nc + kG3 - 1) / kG3, 148 * 8), 128, 0, st, a, sc);
+    if (e != cudaSuccess) return e;
+    e = launch_dep(fo_offsets_kernel, (unsigned)sc.nb, kScanThreads, 0, st, sc, a.host_hdr);
+    if (e != cudaSuccess) return e;
+    return launch_freezeout_emit(a, st);
 }
 
 /* the emit step alone, from the offsets the last launch_freezeout left in the
  * scratch: the elements of a block that did not fit, into a larger buffer */
-void launch_freezeout_emit(const FoArgs &a, cudaStream_t st)
+cudaError_t launch_freezeout_emit(const FoArgs &a, cudaStream_t st)
 {
-    if (!a.elems || a.cap <= 0) return;
+    if (!a.elems || a.cap <= 0) return cudaSuccess;
     const FoScratch sc = carve(a);
     const unsigned grid = (unsigned)std::min((sc.nc + 7) / 8, 148 * 16);
-    if (a.eos.kind == 1) launch_dep(fo_emit_kernel<1>, grid, 128, 0, st, a, sc);
-    else launch_dep(fo_emit_kernel<0>, grid, 128, 0, st, a, sc);
+    if (a.eos.kind == 1) return launch_dep(fo_emit_kernel<1>, grid, 128, 0, st, a, sc);
+    return launch_dep(fo_emit_kernel<0>, grid, 128, 0, st, a, sc);
 }
 
 } // namespace vh

@@ -162,10 +162,10 @@ constexpr int kFoHeaderInts = 4;
 
 /* Runs the whole freezeout block; leaves the elements in a.elems and the
  * cells above e_F and the number of elements in a.host_hdr. */
-void launch_freezeout(const FoArgs &a, cudaStream_t s);
+cudaError_t launch_freezeout(const FoArgs &a, cudaStream_t s);
 /* nz = 1: write the eta ghost planes of one padded field plane (ncz = 5) */
 void launch_eta_ghost_fill(double *plane, int nx, int ny, int ncx, int ncy, cudaStream_t s);
-void launch_freezeout_emit(const FoArgs &a, cudaStream_t s);
+cudaError_t launch_freezeout_emit(const FoArgs &a, cudaStream_t s);
 void launch_cornelius_batch(int dim, const double *cubes, int n, double v0, const double *dx,
                             double *slots, int *counts, int *err, cudaStream_t st);
 size_t freezeout_scratch_ints(int nx, int ny, int nz);

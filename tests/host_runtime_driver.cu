@@ -314,6 +314,21 @@ void regrow_failure()
     vh_event_destroy(ev);
 }
 
+/* a block of whose four kernels one cannot be launched reports it, and the
+ * next block starts from a clean header */
+void chain_failure()
+{
+    for (const char *k : {"fo_open_kernel", "fo_count3_kernel", "fo_offsets_kernel", "fo_emit_kernel"}) {
+        vh_event *ev = make(9, 8, 1);
+        good_block(ev, 3, 1);
+        fail_kernel = k;
+        expect(vh_event_freezeout_launch(ev) != VH_OK, "the failed launch is reported");
+        good_block(ev, 4, 2);
+        expect(!list_overrun, "the crossed-cube counter starts at zero");
+        vh_event_destroy(ev);
+    }
+}
+
 void step(vh_event *ev, const char *what) { expect(vh_event_step(ev, 2) == VH_OK, what); }
 
 } // namespace
@@ -322,7 +337,7 @@ int main(int argc, char **argv)
 {
     const std::map<std::string, void (*)()> all = {
         {"error_cleared", error_cleared},
-        {"setup_rollback", setup_rollback}, {"regrow_failure", regrow_failure}};
+        {"setup_rollback", setup_rollback}, {"regrow_failure", regrow_failure}, {"chain_failure", chain_failure}};
     auto it = argc > 1 ? all.find(argv[1]) : all.end();
     if (it == all.end()) return 2;
     it->second();
