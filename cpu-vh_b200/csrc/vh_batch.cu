@@ -345,10 +345,9 @@ int build_line_tiles(vh_batch *b)
         BTRY(cudaMalloc(&b->ltiles[d], f[d].size() * sizeof(int4)));
         BTRY(cudaMemcpy(b->ltiles[d], f[d].data(), f[d].size() * sizeof(int4), cudaMemcpyHostToDevice));
         vh::BatchKernel k = vh::batch_lines_kernel(b->nq, b->eos_kind, d + 1);
-        BTRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->lsmem[d]));
         /* shared memory for 4 resident blocks, the rest to L1 (the EoS table) */
         const int pct = (int)((4 * (b->lsmem[d] + sizeof(vh::StageArgs) + 1024) * 100 + 228 * 1024 - 1) / (228 * 1024));
-        BTRY(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, std::min(pct, 100)));
+        BTRY(vh::smem_opt_in((const void *)k, b->lsmem[d], pct));
     }
     return VH_OK;
 }

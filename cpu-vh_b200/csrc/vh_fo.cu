@@ -774,14 +774,13 @@ static cudaError_t launch_dep(void (*kernel)(P...), unsigned grid, unsigned bloc
 
 static cudaError_t launch_count4(const FoArgs &a, FoScratch sc, cudaStream_t st)
 {
-    static int blocks = [] {
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaFuncSetAttribute(fo_count4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Count4Shared));
-        int per_sm = 1;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fo_count4_kernel, 128, sizeof(Count4Shared));
-        return sms * (per_sm > 0 ? per_sm : 1);
+    const cudaError_t e = smem_opt_in((const void *)fo_count4_kernel, sizeof(Count4Shared), -1);
+    if (e != cudaSuccess) return e;
+    static const int blocks = [] {      /* of one wave: the same on every device */
+        int per_sm = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fo_count4_kernel, 128, sizeof(Count4Shared)) != cudaSuccess)
+            cudaGetLastError();
+        return 148 * std::max(1, per_sm);
     }();
     const long long need = ((long long)sc.nc + kG4 - 1) / kG4;
     const unsigned grid = (unsigned)(need < blocks ? (need > 0 ? need : 1) : blocks);

@@ -48,6 +48,13 @@ struct InitArgs {
 };
 
 void launch_init(const InitArgs &a, cudaStream_t s);
+
+/* Raises a kernel's dynamic shared memory limit on the current device to at
+ * least bytes, and its carveout to pct percent with it (pct < 0: left as it is).
+ * The limit belongs to the kernel and the device, and kernels take sizes that
+ * depend on the lattice: it is never lowered, whatever the order of the calls
+ * and their threads, so that a launch allowed once stays allowed (vh_kt.cu). */
+cudaError_t smem_opt_in(const void *kernel, size_t bytes, int pct);
 /* interior arrays (nplanes x nx*ny*nz) -> the interior of padded planes */
 void launch_scatter_interior(const double *in, double *out, int nplanes, long long L, int nx, int ny, int nz,
                              int ncx, int ncy, cudaStream_t s);

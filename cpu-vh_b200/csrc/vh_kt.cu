@@ -22,6 +22,9 @@
  */
 #include <cuda_runtime.h>
 #include <cstdlib>
+#include <map>
+#include <mutex>
+#include <utility>
 #include "vh_stage_kernels.cuh"
 
 namespace vh {
@@ -212,6 +215,23 @@ void launch_scatter_interior(const double *in, double *out, int nplanes, long lo
     dim3 block(32, 4, 1);
     dim3 grid((nx + 31) / 32, (ny + 3) / 4, nz);
     scatter_interior_kernel<<<grid, block, 0, s>>>(in, out, nplanes, L, nx, ny, nz, ncx, ncy);
+}
+
+cudaError_t smem_opt_in(const void *kernel, size_t bytes, int pct)
+{
+    static std::mutex mu;
+    static std::map<std::pair<int, const void *>, size_t> limit;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(mu);
+    size_t &have = limit[{dev, kernel}];
+    if (bytes <= have) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return e;
+    if (pct >= 0) e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct < 100 ? pct : 100);
+    if (e == cudaSuccess) have = bytes;
+    return e;
 }
 
 void launch_init(const InitArgs &a, cudaStream_t s)

@@ -173,14 +173,9 @@ template <int NQ, int EOS, int DIR>
 static void launch_flux_slopes(const StageArgs &a, dim3 grid, dim3 block, cudaStream_t s)
 {
     constexpr size_t bytes = sizeof(double) * FluxTile<DIR, 32, 4>::kDoubles(NQ);
-    static const bool attr = [] {
-        cudaFuncSetAttribute(kt_flux_slopes_kernel<NQ, EOS, DIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)bytes);
-        cudaFuncSetAttribute(kt_flux_slopes_kernel<NQ, EOS, DIR>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             (int)((VH_STAGE_MIN_BLOCKS * (bytes + 1024) * 100 + 228 * 1024 - 1) / (228 * 1024)));
-        return true;
-    }();
-    (void)attr;
+    if (smem_opt_in((const void *)kt_flux_slopes_kernel<NQ, EOS, DIR>, bytes,
+                    (int)((VH_STAGE_MIN_BLOCKS * (bytes + 1024) * 100 + 228 * 1024 - 1) / (228 * 1024))) != cudaSuccess)
+        return;     /* the error stays for the caller's cudaGetLastError() */
     kt_flux_slopes_kernel<NQ, EOS, DIR><<<grid, block, bytes, s>>>(a);
 }
 
@@ -199,20 +194,16 @@ static void launch_flux_lines(const StageArgs &a, cudaStream_t s)
     using G = FluxLines<DIR>;
     const int nd = (DIR == 1) ? a.nx : (DIR == 2) ? a.ny : a.nz;
     const size_t bytes = sizeof(double) * 2 * NQ * (size_t)G::plane(nd);
-    static size_t attr_bytes = 0;
-    if (bytes > attr_bytes) {
-        cudaFuncSetAttribute(kt_flux_lines_kernel<NQ, EOS, DIR, MB, UNR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)bytes);
-        /* shared memory for MB resident blocks (1 KB reserved per block) out
-         * of 228 KB, and the rest of the SM's 256 KB left to L1, which holds
-         * the EoS table of the root solves; VH_CARVEOUT overrides (percent) */
-        int pct = (int)((MB * (bytes + 1024) * 100 + 228 * 1024 - 1) / (228 * 1024));
-        if (pct > 100) pct = 100;
-        if (const char *e = getenv("VH_CARVEOUT")) pct = atoi(e);
-        cudaFuncSetAttribute(kt_flux_lines_kernel<NQ, EOS, DIR, MB, UNR>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             pct);
-        attr_bytes = bytes;
-    }
+    /* shared memory for MB resident blocks (1 KB reserved per block) out of
+     * 228 KB, and the rest of the SM's 256 KB left to L1, which holds the EoS
+     * table of the root solves; VH_CARVEOUT overrides (percent) */
+    static const int forced = [] {
+        const char *e = getenv("VH_CARVEOUT");
+        return e ? atoi(e) : -1;
+    }();
+    const int pct = forced >= 0 ? forced : (int)((MB * (bytes + 1024) * 100 + 228 * 1024 - 1) / (228 * 1024));
+    if (smem_opt_in((const void *)kt_flux_lines_kernel<NQ, EOS, DIR, MB, UNR>, bytes, pct) != cudaSuccess)
+        return;     /* the error stays for the caller's cudaGetLastError() */
     const long long runs = (long long)nd * G::bundles(a.nx, a.ny, a.nz);
     const unsigned blocks = (unsigned)((runs + G::PB - 1) / G::PB);
     launch_pdl(kt_flux_lines_kernel<NQ, EOS, DIR, MB, UNR>, dim3(blocks), dim3(128), bytes, s, a);

@@ -331,13 +331,60 @@ void chain_failure()
 
 void step(vh_event *ev, const char *what) { expect(vh_event_step(ev, 2) == VH_OK, what); }
 
+/* short lines need more than 48 KB: on every device, in any order of lengths */
+void opt_in_devices()
+{
+    for (int d : {0, 1}) {
+        cudaSetDevice(d);
+        vh_event *a = make(41, 37, 5), *b = make(41, 37, 9), *c = make(21, 19, 4);
+        step(b, "longer lines");
+        step(a, "short lines");
+        step(b, "longer lines again");
+        block_total = 2;
+        expect(vh_event_freezeout(c, nullptr, nullptr) == VH_OK, "3+1D block");
+        for (vh_event *e : {a, b, c}) vh_event_destroy(e);
+    }
+}
+
+/* the smaller of two first opt-ins, made at the same time, takes effect last */
+void opt_in_threads()
+{
+    vh_event *a = make(41, 37, 5), *b = make(41, 37, 9);
+    small_attr = "kt_flux_lines_kernel";
+    std::thread tb([&] { step(b, "longer lines"); });
+    std::this_thread::sleep_for(std::chrono::milliseconds(100));
+    step(a, "short lines");
+    std::this_thread::sleep_for(std::chrono::milliseconds(200));
+    step(a, "short lines again");
+    tb.join();
+    small_attr.clear();
+    step(b, "longer lines again");
+    vh_event_destroy(a);
+    vh_event_destroy(b);
+}
+
+/* a batch created later with longer lines leaves the earlier one's opt-in */
+void opt_in_batches()
+{
+    vh_event *a = make(41, 37, 5), *b = make(41, 37, 20);
+    vh_batch *ba = nullptr, *bb = nullptr;
+    expect(vh_batch_create(&a, 1, &ba) == VH_OK, "batch of short lines");
+    expect(vh_batch_create(&b, 1, &bb) == VH_OK, "batch of longer lines");
+    expect(vh_batch_step(bb, 1) == VH_OK, "longer lines");
+    expect(vh_batch_step(ba, 1) == VH_OK, "short lines");
+    vh_batch_destroy(ba);
+    vh_batch_destroy(bb);
+    vh_event_destroy(a);
+    vh_event_destroy(b);
+}
 } // namespace
 
 int main(int argc, char **argv)
 {
     const std::map<std::string, void (*)()> all = {
         {"error_cleared", error_cleared},
-        {"setup_rollback", setup_rollback}, {"regrow_failure", regrow_failure}, {"chain_failure", chain_failure}};
+        {"setup_rollback", setup_rollback}, {"regrow_failure", regrow_failure}, {"chain_failure", chain_failure},
+        {"opt_in_devices", opt_in_devices}, {"opt_in_threads", opt_in_threads}, {"opt_in_batches", opt_in_batches}};
     auto it = argc > 1 ? all.find(argv[1]) : all.end();
     if (it == all.end()) return 2;
     it->second();

@@ -26,7 +26,7 @@ def driver(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("scenario", ["error_cleared", "regrow_failure", "setup_rollback", "chain_failure"])
+@pytest.mark.parametrize("scenario", ["error_cleared", "regrow_failure", "setup_rollback", "chain_failure", "opt_in_devices", "opt_in_threads", "opt_in_batches"])
 def test_scenario(driver, scenario):
     env = {k: v for k, v in os.environ.items() if not k.startswith("VH_")}
     r = subprocess.run([driver, scenario], env=env, capture_output=True, text=True, timeout=120)
