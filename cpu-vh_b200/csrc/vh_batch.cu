@@ -209,6 +209,7 @@ struct vh_batch {
     int n_ftiles[3] = {};
     int4 *fltiles[3] = {};           /* mixed precision: face line blocks per axis */
     int n_fltiles[3] = {};
+    bool lines = false;              /* FP64: the flux runs over line pieces */
     int4 *ltiles[3] = {};            /* FP64: line blocks (member, block) per axis */
     int n_ltiles[3] = {};
     size_t lsmem[3] = {};            /* their dynamic shared memory */
@@ -329,6 +330,8 @@ bool batch_lines_on()
  * blocks in member order (eta: the 3+1D members) */
 int build_line_tiles(vh_batch *b)
 {
+    b->lines = batch_lines_on();
+    for (const vh_event *ev : b->mem) b->lines &= vh::limiter_ranged(ev->cfg.theta);
     std::vector<int4> f[3];
     for (size_t m = 0; m < b->mem.size(); ++m) {
         const vh_config &c = b->mem[m]->cfg;
@@ -470,7 +473,7 @@ void launch_stage(vh_batch *b, int stage, const vh_batch_tuning &t, vh::StageMar
          * single events (the tile shape of these phases is then unused) */
         const bool flux = phase >= VH_PHASE_FLUX_X && phase <= VH_PHASE_FLUX_ETA;
         if (flux && b->mixed) launch_face(b, stage, phase - VH_PHASE_FLUX_X + 1);
-        else if (flux && batch_lines_on()) launch_lines(b, stage, phase - VH_PHASE_FLUX_X + 1);
+        else if (flux && b->lines) launch_lines(b, stage, phase - VH_PHASE_FLUX_X + 1);
         else launch_phase(b, stage, phase, t.tile_x[phase], t.persistent[phase]);
         if (m) { m->phase[m->n] = phase; cudaEventRecord(m->ev[++m->n], b->stream); }
     };

@@ -126,6 +126,8 @@ static inline vh::DevEos dev_eos(const vh_event *ev)
         if (!(E.cs2_third_hi >= 0x1p-60) || !E.ranged) E.direct = 0;
         else E.direct = hi - lo < E.direct ? hi - lo : E.direct;
     }
+    /* (an earlier t0 would take t^2 M3^2 below what state_ranged's argument allows for) */
+    if (!vh::limiter_ranged(ev->cfg.theta) || ev->cfg.t0 < 0x1p-60) { E.direct = 0; E.ranged = 0; }
     E.pq.keys = ev->powf.keys;
     E.pq.vals = ev->powf.vals;
     E.pq.bucket = ev->powf.bucket;

@@ -38,6 +38,17 @@ struct StageArgs {
     DevErr err;
 };
 
+/* Whether the branch-free limiter and the range argument of the branch-free
+ * quotients (limited, state_ranged) hold for this theta.  With an infinite one
+ * the difference of equal values is not a number, whose sign bit the hardware
+ * sets and the reference's comparisons do not see; one below 2^-20 makes half
+ * slopes smaller than the argument allows for. */
+inline bool limiter_ranged(double theta)
+{
+    const double a = theta < 0 ? -theta : theta;
+    return a == 0 || (a >= 0x1p-20 && a < 0x1p100);
+}
+
 /* Interior initial condition -> padded state (DynamicalVariables.cpp:169-218
  * and the ghost faces). */
 struct InitArgs {

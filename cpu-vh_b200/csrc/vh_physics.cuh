@@ -141,10 +141,10 @@ __device__ __forceinline__ double approx_deriv(double th, double x, double y, do
  * bits and the minimum of their magnitudes from their bit patterns (which
  * order as the magnitudes do): all negative -> -m, none negative -> m, else
  * +0.  A difference of -0 counts as negative here and not there, but then m = 0
- * and both give +0 (the FMA adds +0).  A NaN loses against a number in the
- * integer minimum, as in fmin.  (With infinite differences of opposite sign
- * approx_deriv gives NaN and this 0 or NaN; the state is then no state: its
- * root solve raises the error either way.)  one: the high word of the factor
+ * and both give +0 (the FMA adds +0).  theta is finite (limiter_ranged), so a
+ * difference is a NaN only where a value is none or infinite; its sign, which
+ * counts here and not there, may then give another slope, but the state is no
+ * state and its step raises the error either way.  one: the high word of the factor
  * on m, 0x3ff00000 for 1, 0x3fe00000 for 1/2 (RN(m/2) as approx_deriv / 2). */
 __device__ __forceinline__ double limited(double th, double x, double y, double z, int one)
 {

@@ -393,7 +393,7 @@ static void launch_stage_t(const StageArgs &a, cudaStream_t s, StageMarks *m)
             mark(2);
             if (z) { launch_pdl(kt_flux_face_kernel<NQ, EOS, 3>, face_grid<3>(a), fb, 0, s, a); mark(3); }
         }
-    } else if (flux_staged() && flux_form() != 0) {
+    } else if (flux_staged() && flux_form() != 0 && limiter_ranged(a.theta)) {
         const dim3 g3((a.nx + 31) / 32, a.ny, (a.nz + 3) / 4);
         if (flux_form() == 2) {
             launch_flux_lines<NQ, EOS, 1, 4, 3>(a, s);
