@@ -226,18 +226,20 @@ __device__ __forceinline__ double e_newton_table_body(const DevEos &E, double eP
 }
 
 /* the same from iterate e0 of iteration j0 on, out of line: a solve that is
- * still going after the few iterations it usually takes */
-static __device__ __noinline__ double e_newton_rest(const DevEos &E, double e0, int j0, double ePrev, double M0, double M,
-                                                    double Pi, bool &bad)
+ * still going after the few iterations it usually takes.  It gives up (false)
+ * where energy_direct's own loop does: a solve that ends in the bisection, which
+ * may run for a second, is then the plain form's alone and not run twice */
+constexpr int kDirectIters = 100;
+static __device__ __noinline__ bool e_newton_rest(const DevEos &E, double e0, int j0, double M0, double M, double Pi, double &e)
 {
-    for (int j = j0; j < 10000; ++j) {
+    for (int j = j0; j < kDirectIters; ++j) {
         bool nan_step, conv;
-        double e = e_newton_iter(E, e0, M0, M, Pi, nan_step, conv);
-        if (nan_step) { bad = true; return ePrev; }
-        if (conv) return e;
+        e = e_newton_iter(E, e0, M0, M, Pi, nan_step, conv);
+        if (nan_step) return false;
+        if (conv) return true;
         e0 = e;
     }
-    return e_bisect_table(E, ePrev, M0, M, Pi);
+    return false;
 }
 
 /* The root solve as a call (one copy of the loop for a long kernel whose
@@ -362,14 +364,12 @@ __device__ __forceinline__ bool energy_direct(const DevEos &E, const double (&M0
         for (int j = 0; ok; ++j) {
             if (REST && j == 8) {
                 /* few lanes are left, and of those mostly one state */
-                bool bad = false;
 #pragma unroll
                 for (int s = 0; s < N; ++s)
-                    if (!done[s]) ef[s] = e_newton_rest(E, e0[s], j, ePrev, M0[s], M[s], Pi[s], bad);
-                ok = !bad;
+                    if (ok && !done[s]) ok = e_newton_rest(E, e0[s], j, M0[s], M[s], Pi[s], ef[s]);
                 break;
             }
-            if (j == 100) { ok = false; break; }
+            if (j == kDirectIters) { ok = false; break; }
             bool all = true;
 #pragma unroll
             for (int s = 0; s < N; ++s) {
