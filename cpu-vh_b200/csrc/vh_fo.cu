@@ -333,7 +333,13 @@ __device__ __forceinline__ void put_count(const FoScratch &sc, int c, int ne)
  * calculate_normal (cornelius.cpp:478-617) run a line per lane, added in the
  * reference's order through width-8 shuffles: the same elements. */
 constexpr int kG3 = 16;                       /* cubes per 128-thread block */
-constexpr int kC3Lines = 12, kC3Polys = 4;     /* 6 squares x 2 lines; a polygon has at least 3 */
+/* 6 squares x 2 lines.  chain_polygons begins a polygon while three lines are
+ * left and puts at least one into it: ten at most, as many as a slot holds
+ * (closed ones are four; none of 4 * 10^7 random cubes, corners on and next to
+ * the threshold and edges down to the matching tolerance 1e-10 among them, gave
+ * more) */
+constexpr int kC3Lines = 12, kC3Polys = 10;
+static_assert(kC3Polys <= cor::kMaxElements, "a cube's elements fit its slot");
 struct Count3Shared {
     double p[kG3][kC3Lines][2][4];
     double out[kG3][kC3Lines][4];
