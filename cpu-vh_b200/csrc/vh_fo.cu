@@ -22,6 +22,34 @@
  * scan and a compaction of flags between gather, classification and count,
  * the same block was thirteen launches: 62 us of device time on a 33x29
  * event against 33.)
+ *
+ * The count kernels (fo_count3_kernel, fo_count4_kernel) restate parts of the
+ * Cornelius subroutine, as vh_cornelius.cuh restates all of it: MODIFIED VERSION
+ * of 2026, its polygon and polyhedron sums spread over a group of lanes, with
+ * the same arithmetic.  The original copyright and permission notice follows;
+ * this file is distributed under the same terms.
+ *
+ * cornelius version 1.3: Copyright 2012, Pasi Huovinen
+ *
+ * This subroutine is aimed to be used as a part of the fluid dynamical
+ * models of the heavy-ion physics community. Permission to use it for
+ * any purpose except for any commercial purpose is granted, provided
+ * that any publication cites the paper describing the algorithm:
+ * P. Huovinen and H. Petersen, arXiv:1206.3371 [nucl-th].
+ *
+ * Permission to distribute this subroutine is granted, provided that no
+ * fee is charged, and that this copyright and permission notice appear
+ * in all the copies. Permission to modify this subroutine is granted
+ * provided that the modified subroutine is made publicly available
+ * latest when any results obtained using the modified subroutine are
+ * published, the modified subroutine is distributed under terms similar
+ * to this notice, and the modified code carries both the original
+ * copyright notice and notices stating that you modified it, and a
+ * relevant date/year.
+ *
+ * This program is distributed in the hope that it will be useful, but
+ * WITHOUT ANY WARRANTY; without even the implied warranty of FITNESS FOR
+ * A PARTICULAR PURPOSE.
  */
 #include <cuda_runtime.h>
 #include <algorithm>
