@@ -175,7 +175,7 @@ constexpr int kFoSlotDoubles = 80;
  * for the stream, 10 us of a 33x29 event's block */
 constexpr int kFoHostElems = 512;
 
-/* the freezeout scratch ends with its header, zero before the first block */
+/* the freezeout scratch ends with its header; its counters are zero before a block */
 constexpr int kFoHeaderInts = 4;
 
 /* Runs the whole freezeout block; leaves the elements in a.elems and the

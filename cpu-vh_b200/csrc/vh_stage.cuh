@@ -4,9 +4,11 @@
  *
  * Every body takes the stage's arguments by reference and the cell it owns;
  * the arithmetic is the reference's, operation for operation, in FP64 with
- * float truncations where the reference has them.  Because both launch forms
- * run these same functions, a cell's result does not depend on which form
- * (fused or phase-split, single event or batch) computed it.
+ * float truncations where the reference has them.  In FP64 a cell's result
+ * therefore does not depend on which launch form (fused or phase-split, single
+ * event or batch) computed it.  The mixed-precision bodies (_m) agree among the
+ * phase-split forms; their fused stage evaluates each face from both sides and
+ * rounds differently.
  */
 #ifndef VH_STAGE_CUH
 #define VH_STAGE_CUH
@@ -437,14 +439,14 @@ struct FluxLines {
     }
 };
 
-/* blk: the block's index among the event's line blocks (runs blk * PB on) */
 /* the face-once flux's line bundles (mixed precision): 8 adjacent x-columns
  * along y and eta (a warp's loads are 4 rows of 64 bytes; 4 columns, 8 rows
  * of 32 bytes, measured 10-11 % slower), the FP64 flux's along x */
 template <int DIR>
 using FaceLinesG = FluxLines<DIR, (DIR == 1) ? VH_FLUX_XW : 8>;
 
-/* What bounds it: a warp's FP64 work is long dependent chains (root solves,
+/* blk: the block's index among the event's line blocks (runs blk * PB on).
+ * What bounds it: a warp's FP64 work is long dependent chains (root solves,
  * then quotients), and 20 warps per SM do not cover them.  The root solves run
  * two states side by side (flow_pair) and the components in groups without a
  * branch per quotient; 131x131x61, one launch: 312 -> 270 us along x, 353 ->

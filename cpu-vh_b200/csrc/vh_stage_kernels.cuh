@@ -277,13 +277,13 @@ static void launch_flux_face_lines(const StageArgs &a, cudaStream_t s)
  * shared memory as the FP64 flux's measured 203/221/245: one face per thread
  * leaves too little work between the block's barriers.  5 blocks per SM of 96
  * registers: 231/235 along x/y. */
-static inline int face_form()
+static inline bool face_lines()
 {
-    static int f = [] {
+    static const bool on = [] {
         const char *e = getenv("VH_FACE_FORM");
-        return (e && e[0] == 't') ? 0 : 4;
+        return !(e && e[0] == 't');
     }();
-    return f;
+    return on;
 }
 
 template <int DIR>
@@ -353,9 +353,12 @@ static void launch_stage_t(const StageArgs &a, cudaStream_t s, StageMarks *m)
     if (!split && stage_faces()) {
         const dim3 gf((a.nx + kFacesTX - 1) / kFacesTX, a.ny, a.nz);
         const dim3 bf(kFacesTX, z ? 7 : 5, 1);
-        /* dependent launch hides the FP64 kernel's launch; the mixed one is
-         * short, and waiting blocks take room from other events' kernels
-         * (three 101^2 events in turn: 206 -> 209 us per 10 steps) */
+        /* dependent launch hides the FP64 kernel's launch.  The mixed one goes
+         * without: both were measured, and it depends on what else is queued.
+         * One event stepping on takes 23.2 us per step with it against 25.5
+         * without (101^2; 161^2: 72.5 against 75.3); passes of a new state and
+         * ten steps queued behind one another over several 101^2 events take
+         * 194 us each with it against 189 without */
         auto go = [&](auto kernel) {
             if constexpr (MIXED) kernel<<<gf, bf, 0, s>>>(a);
             else launch_pdl(kernel, gf, bf, 0, s, a);
@@ -379,7 +382,7 @@ static void launch_stage_t(const StageArgs &a, cudaStream_t s, StageMarks *m)
     launch_pdl(kt_source_kernel<NQ, EOS, MIXED>, gflat, dim3(128), 0, s, a);
     mark(0);
     if constexpr (MIXED) {
-        if (face_form() != 0) {
+        if (face_lines()) {
             launch_flux_face_lines<NQ, EOS, 1, 4>(a, s);
             mark(1);
             launch_flux_face_lines<NQ, EOS, 2, 4>(a, s);

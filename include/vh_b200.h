@@ -158,7 +158,9 @@ int vh_event_freezeout_launch(vh_event *ev);
 int vh_event_freezeout_finish(vh_event *ev, int *n_elements, int *n_above);
 
 /* Copy the elements of the last freezeout block to host memory, VH_FO_COLUMNS
- * doubles per element.  Returns VH_ERR_CAPACITY if cap_elements is too small. */
+ * doubles per element.  Returns VH_ERR_CAPACITY if cap_elements is too small, and
+ * VH_ERR_STATE after a block whose element buffer could not grow (its
+ * vh_event_freezeout_finish failed) until the next block. */
 int vh_event_fetch_surface(vh_event *ev, double *host_out, int cap_elements, int *n_elements);
 
 /* Kernel launches one vh_event_step(ev, 1) issues (2 RK stages; a stage is
