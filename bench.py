@@ -62,9 +62,9 @@ def phase_words(nq):
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) from the
 # ncu captures kept in profiles/kt_flux_lines_kernel_glauber_131x131x61.md
 # (FP64: mean of the x, y, eta launches) and
-# profiles/kt_flux_face_kernel_glauber_131x131x61_mixed.md (mixed)
+# profiles/kt_flux_face_lines_kernel_glauber_131x131x61_mixed.md (mixed)
 NCU_TRAFFIC = {("glauber_3p1d", "fp64", "flux"): 378.96e6, ("glauber_3p1d", "fp64", "source"): 318.90e6,
-               ("glauber_3p1d", "mixed", "flux"): 388.30e6, ("glauber_3p1d", "mixed", "source"): 322.01e6}
+               ("glauber_3p1d", "mixed", "flux"): 403.12e6, ("glauber_3p1d", "mixed", "source"): 317.26e6}
 
 
 # FP64 pipe use of the dominant kernel from the same captures: mean over the
@@ -78,9 +78,9 @@ NCU_FP64 = {("glauber_3p1d", "fp64", "flux"): (44.03, 0.1801, 44.37e6)}
 # batched flux launches: DRAM bytes per cell from ncu captures of the same
 # batch cut to its first 64 events (1 312 264 cells), scaled by the cell count
 # (the traffic of a launch is per cell: each member's stencil once), from
-# profiles/kt_batch_kernel_hotspots_64ev_fp64.md and
-# profiles/kt_batch_face_kernel_hotspots_64ev_mixed.md
-NCU_TRAFFIC_PER_CELL = {("fp64", "flux"): 371.7, ("mixed", "flux"): 371.6}
+# profiles/kt_batch_lines_kernel_hotspots_64ev_fp64.md and
+# profiles/kt_batch_face_lines_kernel_hotspots_64ev_mixed.md
+NCU_TRAFFIC_PER_CELL = {("fp64", "flux"): 366.7, ("mixed", "flux"): 389.9}
 
 
 # steps of the mixed-precision error report: the Gubser event's 300 steps
@@ -93,7 +93,7 @@ PRECISION_STEPS = {"gubser_2p1d": 300, "glauber_3p1d": 800}
 
 
 KERNEL_NAMES = {"source": "kt_source_kernel", "flux": "kt_flux_lines_kernel (x, y, eta)",
-                "final": "kt_final_kernel", "fused": "kt_stage_kernel"}
+                "final": "kt_final_kernel", "fused": "kt_stage_faces_kernel"}
 
 
 def parse():
@@ -921,7 +921,8 @@ def run_batch(args, torch, world, rank, barrier, max_over_ranks):
                              "frac": achieved / peak,
                              "traffic": (NCU_TRAFFIC_PER_CELL[(args.precision, dom)] * Ntot
                                          if (args.precision, dom) in NCU_TRAFFIC_PER_CELL else None),
-                             "kernel": ("kt_batch_face_kernel " if mixed and dom == "flux" else "kt_batch_kernel ") + dom,
+                             "kernel": ("kt_batch_kernel " if dom != "flux" else
+                                        "kt_batch_face_lines_kernel " if mixed else "kt_batch_lines_kernel ") + dom,
                              "launches": dom_n,
                              "launch_us": launch_s * 1e6, "algorithmic_bytes": alg_bytes,
                              "share": dom_ms / sum(t for t, _ in kern.values()),
@@ -1092,7 +1093,7 @@ def main():
                            "l2": l2_note},
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                              "frac": achieved / peak, "traffic": traffic,
-                             "kernel": ("kt_flux_face_kernel (x, y, eta)" if mixed and dom == "flux" and
+                             "kernel": ("kt_flux_face_lines_kernel (x, y, eta)" if mixed and dom == "flux" and
                                         ev.launches_per_step() > 2 else KERNEL_NAMES[dom]), "launches": dom_n,
                              "launch_us": launch_s * 1e6, "algorithmic_bytes": alg_bytes,
                              "share": dom_ms / sum(t for t, _ in kern.values()),
